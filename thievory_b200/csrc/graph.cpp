@@ -1070,7 +1070,7 @@ thv_status thv_run(thv_graph *g, thv_algo algo, const thv_run_opts *o,
       s = run_pagerank(g, algo, o, st, &local);
       if (s == THV_OK && out_values) {
         s = pagerank_values(g, (double *)out_values, st);
-        local.d2h_bytes += g->nv * 4;
+        local.d2h_bytes += g->nv * 8;
       }
       break;
     default:
