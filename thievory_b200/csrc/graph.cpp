@@ -366,8 +366,10 @@ void plan_free(thv_graph *g) {
   dev_free(p.d_list_idx);
   dev_free(p.d_vbegin);
   dev_free(p.d_base);
-  dev_free(p.d_tiles);
-  dev_free(p.d_split_parts);
+  for (PrTiles &t : p.tiles) {
+    dev_free(t.d_tiles);
+    dev_free(t.d_split_parts);
+  }
   p = Plan();
 }
 
@@ -685,21 +687,18 @@ thv_status ensure_plan(thv_graph *g) {
   return do_plan(g, nullptr);
 }
 
-// PageRank tiles: <= kTileEdges edges and <= kTileVerts vertices, never
-// crossing a block; a vertex above kSplitDeg is cut into parts of <=
-// kTileEdges edges whose partial sums are combined atomically.
-constexpr uint64_t kTileEdges = 4096;
-constexpr uint64_t kTileVerts = 2048;
-constexpr uint64_t kSplitDeg = 1024;
-
-thv_status build_tiles(thv_graph *g) {
-  Plan &p = g->plan;
-  if (p.tiles_valid) return THV_OK;
+// PageRank tiles within the bounds of kTileShape[kind], never crossing a
+// block; a vertex of more than split_deg edges is cut into parts of at most
+// part_edges edges whose partial sums are combined atomically.
+thv_status build_tiles(thv_graph *g, PrTileKind kind) {
+  const Plan &plan = g->plan;
+  const PrTileShape &sh = kTileShape[kind];
+  PrTiles &p = g->plan.tiles[kind];
+  if (p.valid) return THV_OK;
   p.tiles.clear();
   p.split_parts.clear();
-  p.tiles_hbm_bytes = p.tiles_link_bytes = 0;
-  for (uint32_t bi = 0; bi < p.blocks.size(); bi++) {
-    const Block &b = p.blocks[bi];
+  for (uint32_t bi = 0; bi < plan.blocks.size(); bi++) {
+    const Block &b = plan.blocks[bi];
     uint32_t start = b.vbegin;
     uint64_t edges = 0;
     auto close = [&](uint32_t end) {
@@ -708,19 +707,19 @@ thv_status build_tiles(thv_graph *g) {
     };
     for (uint32_t v = b.vbegin; v < b.vend; v++) {
       const uint64_t d = g->off[v + 1] - g->off[v];
-      if (d > kSplitDeg) {
+      if (d > sh.split_deg) {
         close(v);
-        const uint32_t parts = (uint32_t)((d + kTileEdges - 1) / kTileEdges);
+        const uint32_t parts = (uint32_t)((d + sh.part_edges - 1) / sh.part_edges);
         const uint32_t sidx = (uint32_t)p.split_parts.size();
         p.split_parts.push_back(parts);
         for (uint32_t k = 0; k < parts; k++) {
-          const uint64_t e0 = g->off[v] + (uint64_t)k * kTileEdges;
-          const uint64_t e1 = std::min<uint64_t>(g->off[v + 1], e0 + kTileEdges);
+          const uint64_t e0 = g->off[v] + (uint64_t)k * sh.part_edges;
+          const uint64_t e1 = std::min<uint64_t>(g->off[v + 1], e0 + sh.part_edges);
           p.tiles.push_back(PrTile{e0, e1, v, v + 1, bi, sidx + 1});
         }
         start = v + 1;
         edges = 0;
-      } else if (edges + d > kTileEdges || v - start >= kTileVerts) {
+      } else if (edges + d > sh.edges || v - start >= sh.verts) {
         close(v);
         start = v;
         edges = d;
@@ -729,9 +728,6 @@ thv_status build_tiles(thv_graph *g) {
       }
     }
     close(b.vend);
-    const uint64_t bytes = (b.eend - b.ebegin) * g->esz;
-    if (b.resident) p.tiles_hbm_bytes += bytes;
-    else p.tiles_link_bytes += bytes;
   }
   // Interleave host-block and HBM-block tiles in proportion to their edges.
   // CTAs take tiles in this order from one counter, so the host link stays
@@ -742,7 +738,7 @@ thv_status build_tiles(thv_graph *g) {
     std::vector<PrTile> host, hbm;
     uint64_t eh = 0, er = 0;
     for (const PrTile &t : p.tiles) {
-      if (p.blocks[t.block].resident) { hbm.push_back(t); er += t.eend - t.ebegin; }
+      if (plan.blocks[t.block].resident) { hbm.push_back(t); er += t.eend - t.ebegin; }
       else { host.push_back(t); eh += t.eend - t.ebegin; }
     }
     size_t i = 0, j = 0;
@@ -765,7 +761,7 @@ thv_status build_tiles(thv_graph *g) {
   if (!p.split_parts.empty())
     THV_CUDA(cudaMemcpy(p.d_split_parts, p.split_parts.data(), p.split_parts.size() * 4,
                         cudaMemcpyHostToDevice));
-  p.tiles_valid = true;
+  p.valid = true;
   return THV_OK;
 }
 

@@ -9,12 +9,12 @@
 // :504-681 (push) with PR32_Update_Values_PUSH :846-860; those iterate to a
 // 1e-3 tolerance in FP64 without dangling redistribution.
 //
-// Every iteration streams all edges.  A CTA takes one tile (<= 4096 edges of
-// consecutive vertices inside one edge block), stages the tile's adjacency in
-// shared memory with 16-byte vector loads -- full 128-byte lines whether the
-// block is in HBM or read zero-copy from pinned host memory -- and then
-// gathers (pull) or scatters (push) per edge.  Per-vertex sums are FP64
-// (warp segmented reductions); stored ranks and contributions are FP32.
+// Every iteration streams all edges.  A warp (pull) or a CTA (push) takes one
+// tile (consecutive vertices inside one edge block, at most 480 or 4,096
+// edges), reads the tile's adjacency with 16-byte vector loads -- full
+// 128-byte lines whether the block is in HBM or read zero-copy from pinned
+// host memory -- and gathers (pull) or scatters (push) per edge.  Per-vertex sums are FP64; stored ranks and
+// contributions are FP32.
 // Pull fuses the rank update into the gather: a vertex's sum is complete
 // inside its tile, except high-degree vertices cut into parts, whose last
 // part (atomic counter) finishes the update.
@@ -27,7 +27,7 @@ namespace thv {
 
 constexpr int kPrThreads = 256;
 constexpr int kPrWarps = kPrThreads / 32;
-constexpr int kStageEdges = 4096;  // == kTileEdges of the tiler
+constexpr int kStageEdges = (int)kTileShape[kCtaTiles].edges;
 
 struct PrArgs {
   const PrTile *tiles;
@@ -45,6 +45,8 @@ struct PrArgs {
   uint32_t *tile_ctr;
   uint32_t ntiles, nv, it;
   uint32_t wshift;  // packed weighted edges: the id is e >> wshift
+  uint32_t last;    // last iteration
+  uint32_t draw;    // pull: tiles a warp draws at a time
   double damping, inv_n;
 };
 
@@ -77,7 +79,7 @@ __device__ __forceinline__ uint32_t out_degree(const PrArgs &a, uint32_t v) {
 __device__ __forceinline__ double finish_vertex(const PrArgs &a, uint32_t v,
                                                 double sum, double base) {
   const double r = base + a.damping * sum;
-  a.rank[v] = (float)r;
+  if (a.last) a.rank[v] = (float)r;  // only the last iteration's ranks are read
   const uint32_t od = out_degree(a, v);
   a.nxt[v] = od ? (float)(r / (double)od) : 0.f;
   return od ? 0.0 : r;
@@ -116,85 +118,228 @@ __device__ __forceinline__ double block_sum(double x, double *s_red) {
   return t;  // valid in thread 0..31
 }
 
-template <int ESZ>
-__global__ void __launch_bounds__(kPrThreads) pr_pull_kernel(PrArgs a) {
-  __shared__ __align__(16) uint32_t s_e[kStageEdges * (ESZ / 4) + 16];
-  __shared__ double s_acc[kPrWarps][32];
+// Pull gather, one tile per warp.  In-edge graphs hold plain 4-byte ids
+// (CSC), so a tile's edges fill at most kPullSlots slots counted from the
+// start of a 128-byte line: each of a warp's loads covers whole lines, in
+// HBM and over the host link alike.  Each slot is handled twice: striped for the
+// gather (coalesced id loads, kPullPer independent gathers in flight per
+// lane) and blocked for the sums (kPullPer consecutive slots per lane), with
+// the gathered contributions crossing over in the warp's shared memory.
+//
+// A lane adds its consecutive slots one after the other in FP64 and closes a
+// row's sum at the row's end; rows that cross a lane's span are combined by
+// one segmented warp reduction per tile.  Nothing in the loop waits for
+// another warp, and the ids of the warp's next tile load during the sums of
+// this one, so some warps gather while others add.  What bounds it is the
+// gather: one L2 sector per edge through each SM's L1 pipe.
+//
+// Measured per iteration at 4.2 M vertices and 65 M in-edges (RMAT, all in
+// HBM): segmented reduction per 32 edges, one gather per lane in flight
+// (about 30 shuffles per 32 edges, L1 pipe 61% busy) 455 us; these sums on
+// 4,092-edge tiles of a 256-thread CTA, two block barriers per tile (a third
+// of the stalls) 390 us; one tile per warp 287 us (227 G edges/s; 4.3 M edges
+// of 262 K vertices: 62 -> 35 us).  With 60% of the edges over the host link,
+// 2.1 M vertices: 2,690 -> 2,606 us (49.8 GB/s of the 51.5 zero-copy rate;
+// 2,879 us while the loads started at 16-byte words).
+constexpr int kPullPer = 16;                    // slots per lane
+constexpr int kPullSlots = 32 * kPullPer;       // >= kTileShape[kWarpTiles].edges + 31
+constexpr int kPullVec = kPullPer / 4;          // 16-byte words per lane
+constexpr int kPullRows = (int)kTileShape[kWarpTiles].verts;
+static_assert(kTileShape[kWarpTiles].edges + 31 < kPullSlots, "a tile fits the slots from any line offset");
+static_assert(kTileShape[kWarpTiles].split_deg <= kTileShape[kWarpTiles].edges, "rows fit tiles");
+
+struct PullWarp {
+  float4 x[kPullSlots / 4];
+  double sum[kPullRows];         // row sums; zero between tiles
+  uint16_t off[kPullRows + 2];   // first slot of each row
+  uint16_t row[32];              // row of each lane's first slot
+};
+
+// Position of 16-byte word v of the contributions in shared memory: striped
+// writes (consecutive words) and blocked reads (every kPullVec-th word) both
+// touch all banks once per eight lanes.
+__device__ __forceinline__ uint32_t pull_slot(uint32_t v) { return v ^ ((v >> 3) & 7u); }
+
+// The 128-byte line of a tile's first edge, the 16-byte words from there to
+// its last edge, and the slot of its first edge.
+struct PullSpan {
+  uintptr_t a0;
+  uint32_t nvec, p0;
+};
+__device__ __forceinline__ PullSpan pull_span(const PrArgs &a, const PrTile &t) {
+  const uintptr_t s0 = (uintptr_t)__ldg(a.blk_base + t.block) + (uintptr_t)t.ebegin * 4;
+  const uintptr_t a0 = s0 & ~(uintptr_t)127;
+  return {a0, (uint32_t)((s0 + (uintptr_t)(t.eend - t.ebegin) * 4 - a0 + 15) / 16),
+          (uint32_t)(s0 - a0) / 4};
+}
+
+// This lane's striped ids of the words [first, first + 32 * kPullVec).
+__device__ __forceinline__ void pull_ids(const PullSpan &s, uint32_t first, uint4 (&q)[kPullVec]) {
+  const unsigned long long stream = l2_evict_first();
+#pragma unroll
+  for (int k = 0; k < kPullVec; k++) {
+    const uint32_t v = first + 32u * k + lane_id();
+    q[k] = v >= s.p0 / 4 && v < s.nvec ? ld_stream_v4(s.a0 + 16u * v, stream) : make_uint4(0, 0, 0, 0);
+  }
+}
+
+// Their contributions; 0 outside the slots [p0, p1).
+__device__ __forceinline__ void pull_gather(const PrArgs &a, uint32_t first, uint32_t p0, uint32_t p1,
+                                            const uint4 (&q)[kPullVec], float (&x)[kPullVec][4]) {
+#pragma unroll
+  for (int k = 0; k < kPullVec; k++) {
+    const uint32_t id[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
+    const uint32_t p = 4u * (first + 32u * k + lane_id());
+#pragma unroll
+    for (int j = 0; j < 4; j++) x[k][j] = p + j >= p0 && p + j < p1 ? __ldg(a.cur + id[j]) : 0.f;
+  }
+}
+
+__global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
+  __shared__ PullWarp s_warp[kPrWarps];
   __shared__ double s_red[kPrWarps];
-  __shared__ uint32_t s_tile;
-  const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
+  PullWarp &s = s_warp[threadIdx.x >> 5];
+  const unsigned lane = lane_id();
   const double base = (1.0 - a.damping) * a.inv_n + a.damping * ldcg(a.dang + a.it) * a.inv_n;
   double dsum = 0.0;
-  for (;;) {
-    if (threadIdx.x == 0) s_tile = atomicAdd(a.tile_ctr + a.it, 1u);
-    __syncthreads();
-    const uint32_t ti = s_tile;
-    if (ti >= a.ntiles) break;
-    const PrTile t = a.tiles[ti];
-    const uint32_t shift = stage_tile<ESZ>(a, t, s_e);
-    __syncthreads();
-    if (t.split) {
-      const uint32_t cnt = (uint32_t)(t.eend - t.ebegin);
-      double part = 0.0;
-      for (uint32_t i = threadIdx.x; i < cnt; i += blockDim.x)
-        part += (double)__ldg(a.cur + staged_id<ESZ>(s_e, shift + i, a.wshift));
-      part = block_sum(part, s_red);
-      if (threadIdx.x == 0) {
-        const uint32_t s = t.split - 1;
-        atomicAdd(a.split_acc + s, part);
-        __threadfence();
-        const uint32_t done = atomicAdd(a.split_done + s, 1u);
-        if (done + 1 == __ldg(a.split_parts + s)) {
-          __threadfence();
-          const unsigned long long bits =
-              atomicExch(reinterpret_cast<unsigned long long *>(a.split_acc + s), 0ull);
-          a.split_done[s] = 0;
-          dsum += finish_vertex(a, t.vbegin, __longlong_as_double((long long)bits), base);
+  for (uint32_t r = lane; r < (uint32_t)kPullRows; r += 32) s.sum[r] = 0.0;
+  // tiles come from a counter, a.draw at a time
+  uint32_t *ctr = a.tile_ctr + a.it;
+  uint32_t ti = 0;
+  if (lane == 0) ti = atomicAdd(ctr, a.draw);
+  ti = __shfl_sync(kFull, ti, 0);
+  uint32_t left = a.draw;
+  PrTile t{};
+  PullSpan sp{};
+  uint4 q[kPullVec];
+  if (ti < a.ntiles) {
+    t = a.tiles[ti];
+    sp = pull_span(a, t);
+    pull_ids(sp, 0, q);
+  }
+  while (ti < a.ntiles) {
+    uint32_t drawn = 0;
+    if (left == 1 && lane == 0) drawn = atomicAdd(ctr, a.draw);
+    const uint32_t p0 = sp.p0, p1 = p0 + (uint32_t)(t.eend - t.ebegin);
+    const uint32_t nrows = t.vend - t.vbegin;
+    if (!t.split) {
+      for (uint32_t r = lane; r < nrows; r += 32) {
+        const uint32_t o0 = p0 + (uint32_t)(__ldg(a.off + t.vbegin + r) - t.ebegin);
+        const uint32_t o1 = p0 + (uint32_t)(__ldg(a.off + t.vbegin + r + 1) - t.ebegin);
+        s.off[r] = (uint16_t)o0;
+        if (r + 1 == nrows) s.off[nrows] = (uint16_t)o1;
+        if (o1 > o0) {
+          // lanes whose span starts inside this row; the first row with
+          // edges also takes the lanes that start in the empty slots before
+          // it (p0 reaches into the second lane's span)
+          for (uint32_t k = o0 == p0 ? 0u : (o0 + kPullPer - 1) / kPullPer; k * kPullPer < o1; k++)
+            s.row[k] = (uint16_t)r;
         }
-      }
-    } else {
-      const uint32_t nverts = t.vend - t.vbegin;
-      const uint32_t ngroups = (nverts + 31) / 32;
-      for (uint32_t g = warp; g < ngroups; g += kPrWarps) {
-        const uint32_t v = t.vbegin + g * 32 + lane;
-        const bool valid = v < t.vend;
-        uint32_t ls = 0, deg = 0;
-        if (valid) {
-          const uint64_t e0 = __ldg(a.off + v), e1 = __ldg(a.off + v + 1);
-          ls = (uint32_t)(e0 - t.ebegin);
-          deg = (uint32_t)(e1 - e0);
-        }
-        const unsigned incl = warp_incl_scan<unsigned>(deg);
-        const unsigned excl = incl - deg;
-        const unsigned total = __shfl_sync(kFull, incl, 31);
-        s_acc[warp][lane] = 0.0;
-        __syncwarp();
-        for (unsigned k = 0; k < total; k += 32) {
-          const unsigned tt = k + lane;
-          const int o = warp_owner(excl, tt);
-          const unsigned ols = __shfl_sync(kFull, ls, o);
-          const unsigned oex = __shfl_sync(kFull, excl, o);
-          double x = 0.0;
-          int pos = 32;
-          if (tt < total) {
-            x = (double)__ldg(a.cur + staged_id<ESZ>(s_e, shift + ols + (tt - oex), a.wshift));
-            pos = o;
-          }
-#pragma unroll
-          for (int d = 1; d < 32; d <<= 1) {
-            const double y = __shfl_up_sync(kFull, x, d);
-            const int pp = __shfl_up_sync(kFull, pos, d);
-            if (lane >= (unsigned)d && pp == pos) x += y;
-          }
-          const int nxt = __shfl_down_sync(kFull, pos, 1);
-          if ((lane == 31 || nxt != pos) && pos < 32) s_acc[warp][pos] += x;
-          __syncwarp();
-        }
-        if (valid) dsum += finish_vertex(a, v, s_acc[warp][lane], base);
-        __syncwarp();
       }
     }
-    __syncthreads();
+    double acc = 0.0;
+    {
+      float x[kPullVec][4];
+      pull_gather(a, 0, p0, p1, q, x);
+      if (t.split) {
+#pragma unroll
+        for (int k = 0; k < kPullVec; k++)
+          acc += ((double)x[k][0] + (double)x[k][1]) + ((double)x[k][2] + (double)x[k][3]);
+      } else {
+#pragma unroll
+        for (int k = 0; k < kPullVec; k++)
+          s.x[pull_slot(32u * k + lane)] = make_float4(x[k][0], x[k][1], x[k][2], x[k][3]);
+      }
+    }
+    const PrTile c = t;
+    const PullSpan cs = sp;
+    if (--left == 0) {
+      ti = __shfl_sync(kFull, drawn, 0);
+      left = a.draw;
+    } else {
+      ti++;
+    }
+    if (c.split) {
+      // the rest of a long row's part
+      for (uint32_t first = 32 * kPullVec; first < cs.nvec; first += 32 * kPullVec) {
+        float x[kPullVec][4];
+        pull_ids(cs, first, q);
+        pull_gather(a, first, p0, p1, q, x);
+#pragma unroll
+        for (int k = 0; k < kPullVec; k++)
+          acc += ((double)x[k][0] + (double)x[k][1]) + ((double)x[k][2] + (double)x[k][3]);
+      }
+    }
+    if (ti < a.ntiles) {
+      t = a.tiles[ti];
+      sp = pull_span(a, t);
+      pull_ids(sp, 0, q);
+    }
+    if (c.split) {
+      acc = warp_sum(acc);
+      if (lane == 0) {
+        const uint32_t sv = c.split - 1, parts = __ldg(a.split_parts + sv);
+        bool last = parts == 1;
+        if (!last) {
+          atomicAdd(a.split_acc + sv, acc);
+          __threadfence();
+          last = atomicAdd(a.split_done + sv, 1u) + 1 == parts;
+          if (last) {
+            __threadfence();
+            acc = __longlong_as_double((long long)atomicExch(
+                reinterpret_cast<unsigned long long *>(a.split_acc + sv), 0ull));
+            a.split_done[sv] = 0;
+          }
+        }
+        if (last) dsum += finish_vertex(a, c.vbegin, acc, base);
+      }
+      continue;
+    }
+    __syncwarp();  // contributions and row table are in place
+    const uint32_t b0 = kPullPer * lane;  // this lane's span [b0, b0 + kPullPer)
+    uint32_t key = 0x10000u + lane;       // row whose open part this lane holds; else its own
+    if (p1 > p0 && b0 < p1) {
+      uint32_t r = s.row[lane], end = s.off[r + 1];
+      bool open = s.off[r] < b0;  // the row began in an earlier span
+#pragma unroll
+      for (int k = 0; k < kPullVec; k++) {
+        const float4 f = s.x[pull_slot(kPullVec * lane + k)];
+        const float x[4] = {f.x, f.y, f.z, f.w};
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+          const uint32_t p = b0 + 4u * k + j;
+          if (p >= end && p < p1) {
+            s.sum[r] = acc;  // the whole row, or its last open part
+            acc = 0.0;
+            open = false;
+            do r++;
+            while (s.off[r + 1] <= p);
+            end = s.off[r + 1];
+          }
+          acc += (double)x[j];
+        }
+      }
+      if (open || end > b0 + kPullPer) key = r;
+      else s.sum[r] = acc;
+    }
+    __syncwarp();
+    // open parts of one row in neighbouring lanes meet in the first of them,
+    // which adds them to the part of the lane that closed the row (if any)
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const double y = __shfl_down_sync(kFull, acc, d);
+      const uint32_t ky = __shfl_down_sync(kFull, key, d);
+      if (lane + d < 32 && ky == key) acc += y;
+    }
+    const uint32_t kp = __shfl_up_sync(kFull, key, 1);
+    if (key < 0x10000u && (lane == 0 || kp != key)) s.sum[key] += acc;
+    __syncwarp();
+    for (uint32_t r = lane; r < nrows; r += 32) {
+      const double sum = s.sum[r];
+      s.sum[r] = 0.0;
+      dsum += finish_vertex(a, c.vbegin + r, sum, base);
+    }
+    __syncwarp();
   }
   dsum = block_sum(dsum, s_red);
   if (threadIdx.x == 0 && dsum != 0.0) atomicAdd(a.dang + a.it + 1, dsum);
@@ -266,7 +411,6 @@ __global__ void pr_init(PrArgs a, float *c0) {
   __shared__ double s_red[kPrWarps];
   double dsum = 0.0;
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.nv; v += gridDim.x * blockDim.x) {
-    a.rank[v] = (float)a.inv_n;
     const uint32_t od = out_degree(a, v);
     c0[v] = od ? (float)(a.inv_n / (double)od) : 0.f;
     if (!od) dsum += a.inv_n;
@@ -579,9 +723,10 @@ void pagerank_free(thv_graph *g) {
   g->ps = nullptr;
 }
 
-static thv_status ensure_pr_state(thv_graph *g, bool push, uint32_t iters, bool ref) {
+static thv_status ensure_pr_state(thv_graph *g, bool push, uint32_t iters, bool ref,
+                                  const PrTiles &tiles) {
   PrState *&p = g->ps;
-  const size_t nsplit = std::max<size_t>(1, g->plan.split_parts.size());
+  const size_t nsplit = std::max<size_t>(1, tiles.split_parts.size());
   if (p && p->push == push && p->ref == ref && (ref || p->cap_iters >= iters) && p->nsplit == nsplit)
     return THV_OK;
   pagerank_free(g);
@@ -626,11 +771,15 @@ static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, uint32_t iters,
   if (push)
     THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_push_kernel<ESZ>, kPrThreads, 0));
   else
-    THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_pull_kernel<ESZ>, kPrThreads, 0));
+    THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_pull_kernel, kPrThreads, 0));
   const int grid = std::max(1, bpsm) * g->num_sms;
   const int ugrid = std::max(1, std::min<int>(g->num_sms * 8, (int)((g->nv + kPrThreads - 1) / kPrThreads)));
+  // several tiles per draw only while every warp still draws often enough
+  // for the last ones to even out
+  a.draw = std::min(4u, std::max(1u, a.ntiles / (16u * (uint32_t)grid * kPrWarps)));
   for (uint32_t it = 0; it < iters; it++) {
     a.it = it;
+    a.last = it + 1 == iters;
     a.cur = p->d_c[it & 1];
     a.nxt = p->d_c[(it + 1) & 1];
     if (push) {
@@ -638,7 +787,7 @@ static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, uint32_t iters,
       pr_push_update<<<ugrid, kPrThreads, 0, st>>>(a);
       launches += 2;
     } else {
-      pr_pull_kernel<ESZ><<<grid, kPrThreads, 0, st>>>(a);
+      pr_pull_kernel<<<grid, kPrThreads, 0, st>>>(a);
       launches += 1;
     }
     THV_CUDA(cudaGetLastError());
@@ -653,11 +802,12 @@ static thv_status run_pagerank_ref(thv_graph *g, thv_algo algo, const thv_run_op
   const bool push = algo == THV_ALGO_PR_PUSH;
   const uint32_t max_rounds = o && o->pr_iters ? o->pr_iters : 100000u;
   THV_TRY(ensure_plan(g));
-  THV_TRY(build_tiles(g));
-  THV_TRY(ensure_pr_state(g, push, 0, true));
+  THV_TRY(build_tiles(g, kCtaTiles));
+  const PrTiles &tiles = g->plan.tiles[kCtaTiles];
+  THV_TRY(ensure_pr_state(g, push, 0, true, tiles));
   PrState *p = g->ps;
   PrRefArgs a{};
-  a.tiles = g->plan.d_tiles;
+  a.tiles = tiles.d_tiles;
   a.blk_base = g->plan.d_base;
   a.off = g->d_off;
   a.outdeg = g->fmt == THV_FMT_CSC ? g->d_outdeg : nullptr;
@@ -667,10 +817,10 @@ static thv_status run_pagerank_ref(thv_graph *g, thv_algo algo, const thv_run_op
   a.act = p->d_act;
   a.split_acc = p->d_split_acc;
   a.split_done = p->d_split_done;
-  a.split_parts = g->plan.d_split_parts;
+  a.split_parts = tiles.d_split_parts;
   a.tile_ctr = p->d_tile_ctr;
   a.cnt = p->d_cnt;
-  a.ntiles = (uint32_t)g->plan.tiles.size();
+  a.ntiles = (uint32_t)tiles.tiles.size();
   a.nv = (uint32_t)g->nv;
   a.wshift = g->wshift;
   int bpsm = 0;
@@ -680,7 +830,7 @@ static thv_status run_pagerank_ref(thv_graph *g, thv_algo algo, const thv_run_op
     THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, g->esz == 8 ? pr_ref_pull_kernel<8> : pr_ref_pull_kernel<4>, kPrThreads, 0));
   const int grid = std::max(1, bpsm) * g->num_sms;
   const int ugrid = std::max(1, std::min<int>(g->num_sms * 8, (int)((g->nv + kPrThreads - 1) / kPrThreads)));
-  const size_t nsplit = std::max<size_t>(1, g->plan.split_parts.size());
+  const size_t nsplit = std::max<size_t>(1, tiles.split_parts.size());
   uint32_t launches = 0, rounds = 0;
   uint64_t edges = 0;
   THV_CUDA(cudaEventRecord(p->ev0, st));
@@ -738,13 +888,15 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   const uint32_t iters = o && o->pr_iters ? o->pr_iters : 20u;
   const double damping = o && o->pr_damping > 0 ? o->pr_damping : 0.85;
   THV_TRY(ensure_plan(g));
-  THV_TRY(build_tiles(g));
-  THV_TRY(ensure_pr_state(g, push, iters, false));
+  const PrTileKind kind = push ? kCtaTiles : kWarpTiles;
+  THV_TRY(build_tiles(g, kind));
+  const PrTiles &tiles = g->plan.tiles[kind];
+  THV_TRY(ensure_pr_state(g, push, iters, false, tiles));
   PrState *p = g->ps;
   p->iters = iters;
 
   PrArgs a{};
-  a.tiles = g->plan.d_tiles;
+  a.tiles = tiles.d_tiles;
   a.blk_base = g->plan.d_base;
   a.off = g->d_off;
   a.outdeg = g->fmt == THV_FMT_CSC ? g->d_outdeg : nullptr;
@@ -752,10 +904,10 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   a.sum = p->d_sum;
   a.split_acc = p->d_split_acc;
   a.split_done = p->d_split_done;
-  a.split_parts = g->plan.d_split_parts;
+  a.split_parts = tiles.d_split_parts;
   a.dang = p->d_dang;
   a.tile_ctr = p->d_tile_ctr;
-  a.ntiles = (uint32_t)g->plan.tiles.size();
+  a.ntiles = (uint32_t)tiles.tiles.size();
   a.nv = (uint32_t)g->nv;
   a.damping = damping;
   a.inv_n = 1.0 / (double)g->nv;
@@ -765,7 +917,7 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   THV_CUDA(cudaEventRecord(p->ev0, st));
   THV_CUDA(cudaMemsetAsync(p->d_dang, 0, (iters + 1) * 8, st));
   THV_CUDA(cudaMemsetAsync(p->d_tile_ctr, 0, iters * 4, st));
-  const size_t nsplit = std::max<size_t>(1, g->plan.split_parts.size());
+  const size_t nsplit = std::max<size_t>(1, tiles.split_parts.size());
   THV_CUDA(cudaMemsetAsync(p->d_split_acc, 0, nsplit * 8, st));
   THV_CUDA(cudaMemsetAsync(p->d_split_done, 0, nsplit * 4, st));
   const int ugrid = std::max(1, std::min<int>(g->num_sms * 8, (int)((g->nv + kPrThreads - 1) / kPrThreads)));
@@ -784,8 +936,10 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
     stats->device_ms = ms_;
     stats->iterations = iters;
     stats->edges_expanded = g->ne * iters;
-    stats->hbm_edge_bytes = g->plan.tiles_hbm_bytes * iters;
-    stats->link_edge_bytes = g->plan.tiles_link_bytes * iters;
+    uint64_t hbm = 0, link = 0;  // whole blocks: PageRank does not read the small-list cache
+    for (const Block &b : g->plan.blocks) (b.resident ? hbm : link) += (b.eend - b.ebegin) * g->esz;
+    stats->hbm_edge_bytes = hbm * iters;
+    stats->link_edge_bytes = link * iters;
     stats->kernel_launches = launches;
   }
   return THV_OK;

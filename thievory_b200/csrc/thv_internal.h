@@ -43,13 +43,33 @@ struct Block {
   uint64_t dev_elem;      // element offset inside the resident buffer
 };
 
-// Dense-iteration tile (PageRank): a vertex range with <= kTileEdges edges
-// inside one block, or one part of a high-degree vertex ("split" tile).
+// Dense-iteration tile (PageRank): a vertex range with a bounded number of
+// edges inside one block, or one part of a high-degree vertex ("split" tile).
 struct __align__(16) PrTile {
   uint64_t ebegin, eend;
   uint32_t vbegin, vend;
   uint32_t block;
   uint32_t split;  // 0, or 1 + index of the split vertex
+};
+
+// Tile sets, built lazily per plan: sized for one CTA (push, and the
+// reference-semantics kernels) or for one warp (pull).
+enum PrTileKind { kCtaTiles = 0, kWarpTiles = 1 };
+struct PrTileShape {
+  uint64_t edges, verts;  // bounds of a tile
+  uint64_t split_deg;     // a vertex above this is cut into split tiles
+  uint64_t part_edges;    // edges of one split tile
+};
+// Pull keeps a tile's edges in 512 slots counted from a 128-byte line, so
+// up to 31 of them lie before its first edge; its split tiles take up to
+// 2,048 such slots.
+constexpr PrTileShape kTileShape[2] = {{4096, 2048, 1024, 4096}, {480, 128, 480, 2016}};
+struct PrTiles {
+  bool valid = false;
+  std::vector<PrTile> tiles;
+  std::vector<uint32_t> split_parts;  // per split vertex
+  PrTile *d_tiles = nullptr;
+  uint32_t *d_split_parts = nullptr;
 };
 
 constexpr uint64_t kDefaultBlockBytes = 64ull << 20;  // reference PARTITION_SIZE_MB
@@ -79,13 +99,7 @@ struct Plan {
   // access tracking: link bytes per block (device counters) and the flags
   uint32_t flags = 0;
   unsigned long long *d_access = nullptr;
-  // PageRank tiles (built lazily)
-  bool tiles_valid = false;
-  std::vector<PrTile> tiles;
-  std::vector<uint32_t> split_parts;  // per split vertex
-  PrTile *d_tiles = nullptr;
-  uint32_t *d_split_parts = nullptr;
-  uint64_t tiles_hbm_bytes = 0, tiles_link_bytes = 0;
+  PrTiles tiles[2];  // by PrTileKind
 };
 
 // Small-list cache as the kernels see it: lists with 0 < deg < deg_lt whose
@@ -174,7 +188,7 @@ thv_status convert_edge_list(const char *txt, const char *out_path, thv_format f
                              uint64_t *ne_out);  // convert.cu
 void transpose_free(thv_graph *g);
 thv_status ensure_plan(thv_graph *g);
-thv_status build_tiles(thv_graph *g);
+thv_status build_tiles(thv_graph *g, PrTileKind kind);
 void plan_free(thv_graph *g);
 
 thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
