@@ -9,11 +9,11 @@
 // :504-681 (push) with PR32_Update_Values_PUSH :846-860; those iterate to a
 // 1e-3 tolerance in FP64 without dangling redistribution.
 //
-// Every iteration streams all edges.  A warp (pull) or a CTA (push) takes one
-// tile (consecutive vertices inside one edge block, at most 480 or 4,096
-// edges), reads the tile's adjacency with 16-byte vector loads -- full
-// 128-byte lines whether the block is in HBM or read zero-copy from pinned
-// host memory -- and gathers (pull) or scatters (push) per edge.  Per-vertex sums are FP64; stored ranks and
+// Every iteration streams all edges.  A warp (or a CTA: push on large
+// resident graphs) takes one tile, consecutive vertices inside one edge
+// block with at most 480 (4,096) edges, reads the tile's adjacency with 16-byte vector loads -- full 128-byte lines whether the
+// block is in HBM or read zero-copy from pinned host memory -- and gathers
+// (pull) or scatters (push) per edge.  Per-vertex sums are FP64; stored ranks and
 // contributions are FP32.
 // Pull fuses the rank update into the gather: a vertex's sum is complete
 // inside its tile, except high-degree vertices cut into parts, whose last
@@ -141,47 +141,94 @@ __device__ __forceinline__ double block_sum(double x, double *s_red) {
 // of 262 K vertices: 62 -> 35 us).  With 60% of the edges over the host link,
 // 2.1 M vertices: 2,690 -> 2,606 us (49.8 GB/s of the 51.5 zero-copy rate;
 // 2,879 us while the loads started at 16-byte words).
-constexpr int kPullPer = 16;                    // slots per lane
-constexpr int kPullSlots = 32 * kPullPer;       // >= kTileShape[kWarpTiles].edges + 31
-constexpr int kPullVec = kPullPer / 4;          // 16-byte words per lane
-constexpr int kPullRows = (int)kTileShape[kWarpTiles].verts;
-static_assert(kTileShape[kWarpTiles].edges + 31 < kPullSlots, "a tile fits the slots from any line offset");
+constexpr int kPer = 16;              // slots per lane
+constexpr int kSlots = 32 * kPer;     // >= kTileShape[kWarpTiles].edges + 31
+constexpr int kPullVec = kPer / 4;    // 16-byte words of ids per lane
+constexpr int kRows = (int)kTileShape[kWarpTiles].verts;
+static_assert(kTileShape[kWarpTiles].edges + 31 < kSlots, "a tile fits the slots from any line offset");
 static_assert(kTileShape[kWarpTiles].split_deg <= kTileShape[kWarpTiles].edges, "rows fit tiles");
 
-struct PullWarp {
-  float4 x[kPullSlots / 4];
-  double sum[kPullRows];         // row sums; zero between tiles
-  uint16_t off[kPullRows + 2];   // first slot of each row
-  uint16_t row[32];              // row of each lane's first slot
+// Rows of a warp's tile in slot numbers.
+struct WarpRows {
+  uint16_t off[kRows + 2];  // first slot of each row
+  uint16_t row[32];         // row of each lane's first slot
 };
 
-// Position of 16-byte word v of the contributions in shared memory: striped
-// writes (consecutive words) and blocked reads (every kPullVec-th word) both
+// Position of 16-byte word v of per-slot floats in shared memory: striped
+// accesses (consecutive words) and blocked ones (every fourth word) both
 // touch all banks once per eight lanes.
-__device__ __forceinline__ uint32_t pull_slot(uint32_t v) { return v ^ ((v >> 3) & 7u); }
+__device__ __forceinline__ uint32_t slot_word(uint32_t v) { return v ^ ((v >> 3) & 7u); }
 
 // The 128-byte line of a tile's first edge, the 16-byte words from there to
 // its last edge, and the slot of its first edge.
-struct PullSpan {
+struct TileSpan {
   uintptr_t a0;
   uint32_t nvec, p0;
 };
-__device__ __forceinline__ PullSpan pull_span(const PrArgs &a, const PrTile &t) {
-  const uintptr_t s0 = (uintptr_t)__ldg(a.blk_base + t.block) + (uintptr_t)t.ebegin * 4;
+template <int ESZ>
+__device__ __forceinline__ TileSpan tile_span(const PrArgs &a, const PrTile &t) {
+  const uintptr_t s0 = (uintptr_t)__ldg(a.blk_base + t.block) + (uintptr_t)t.ebegin * ESZ;
   const uintptr_t a0 = s0 & ~(uintptr_t)127;
-  return {a0, (uint32_t)((s0 + (uintptr_t)(t.eend - t.ebegin) * 4 - a0 + 15) / 16),
-          (uint32_t)(s0 - a0) / 4};
+  return {a0, (uint32_t)((s0 + (uintptr_t)(t.eend - t.ebegin) * ESZ - a0 + 15) / 16),
+          (uint32_t)(s0 - a0) / ESZ};
 }
 
-// This lane's striped ids of the words [first, first + 32 * kPullVec).
-__device__ __forceinline__ void pull_ids(const PullSpan &s, uint32_t first, uint4 (&q)[kPullVec]) {
+// This lane's striped words [first, first + 32 * N) of a tile's edges.
+template <int ESZ, int N>
+__device__ __forceinline__ void tile_words(const TileSpan &s, uint32_t first, uint4 (&q)[N]) {
   const unsigned long long stream = l2_evict_first();
 #pragma unroll
-  for (int k = 0; k < kPullVec; k++) {
+  for (int k = 0; k < N; k++) {
     const uint32_t v = first + 32u * k + lane_id();
-    q[k] = v >= s.p0 / 4 && v < s.nvec ? ld_stream_v4(s.a0 + 16u * v, stream) : make_uint4(0, 0, 0, 0);
+    q[k] = v >= s.p0 / (16 / ESZ) && v < s.nvec ? ld_stream_v4(s.a0 + 16u * v, stream)
+                                                : make_uint4(0, 0, 0, 0);
   }
 }
+
+// Row table of an unsplit tile whose first edge sits in slot p0.
+__device__ __forceinline__ void tile_rows(const PrArgs &a, const PrTile &t, uint32_t p0, WarpRows &s) {
+  const uint32_t nrows = t.vend - t.vbegin;
+  for (uint32_t r = lane_id(); r < nrows; r += 32) {
+    const uint32_t o0 = p0 + (uint32_t)(__ldg(a.off + t.vbegin + r) - t.ebegin);
+    const uint32_t o1 = p0 + (uint32_t)(__ldg(a.off + t.vbegin + r + 1) - t.ebegin);
+    s.off[r] = (uint16_t)o0;
+    if (r + 1 == nrows) s.off[nrows] = (uint16_t)o1;
+    if (o1 > o0) {
+      // lanes whose span starts inside this row; the first row with edges
+      // also takes the lanes that start in the empty slots before it (p0
+      // reaches into the second lane's span)
+      for (uint32_t k = o0 == p0 ? 0u : (o0 + kPer - 1) / kPer; k * kPer < o1; k++)
+        s.row[k] = (uint16_t)r;
+    }
+  }
+}
+
+// Tiles from the iteration's counter, a.draw at a time per warp: the tile
+// after ti (ask before the work on ti that hides the draw, take after it).
+struct TileDraw {
+  uint32_t left, drawn;
+};
+__device__ __forceinline__ uint32_t first_tile(const PrArgs &a, TileDraw &d) {
+  uint32_t ti = 0;
+  if (lane_id() == 0) ti = atomicAdd(a.tile_ctr + a.it, a.draw);
+  d.left = a.draw;
+  return __shfl_sync(kFull, ti, 0);
+}
+__device__ __forceinline__ void ask_tile(const PrArgs &a, TileDraw &d) {
+  d.drawn = 0;
+  if (d.left == 1 && lane_id() == 0) d.drawn = atomicAdd(a.tile_ctr + a.it, a.draw);
+}
+__device__ __forceinline__ uint32_t take_tile(const PrArgs &a, TileDraw &d, uint32_t ti) {
+  if (--d.left) return ti + 1;
+  d.left = a.draw;
+  return __shfl_sync(kFull, d.drawn, 0);
+}
+
+struct PullWarp {
+  float4 x[kSlots / 4];  // contributions by slot
+  double sum[kRows];     // row sums; zero between tiles
+  WarpRows rows;
+};
 
 // Their contributions; 0 outside the slots [p0, p1).
 __device__ __forceinline__ void pull_gather(const PrArgs &a, uint32_t first, uint32_t p0, uint32_t p1,
@@ -202,41 +249,22 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
   const unsigned lane = lane_id();
   const double base = (1.0 - a.damping) * a.inv_n + a.damping * ldcg(a.dang + a.it) * a.inv_n;
   double dsum = 0.0;
-  for (uint32_t r = lane; r < (uint32_t)kPullRows; r += 32) s.sum[r] = 0.0;
-  // tiles come from a counter, a.draw at a time
-  uint32_t *ctr = a.tile_ctr + a.it;
-  uint32_t ti = 0;
-  if (lane == 0) ti = atomicAdd(ctr, a.draw);
-  ti = __shfl_sync(kFull, ti, 0);
-  uint32_t left = a.draw;
+  for (uint32_t r = lane; r < (uint32_t)kRows; r += 32) s.sum[r] = 0.0;
+  TileDraw draw;
+  uint32_t ti = first_tile(a, draw);
   PrTile t{};
-  PullSpan sp{};
+  TileSpan sp{};
   uint4 q[kPullVec];
   if (ti < a.ntiles) {
     t = a.tiles[ti];
-    sp = pull_span(a, t);
-    pull_ids(sp, 0, q);
+    sp = tile_span<4>(a, t);
+    tile_words<4>(sp, 0, q);
   }
   while (ti < a.ntiles) {
-    uint32_t drawn = 0;
-    if (left == 1 && lane == 0) drawn = atomicAdd(ctr, a.draw);
+    ask_tile(a, draw);
     const uint32_t p0 = sp.p0, p1 = p0 + (uint32_t)(t.eend - t.ebegin);
     const uint32_t nrows = t.vend - t.vbegin;
-    if (!t.split) {
-      for (uint32_t r = lane; r < nrows; r += 32) {
-        const uint32_t o0 = p0 + (uint32_t)(__ldg(a.off + t.vbegin + r) - t.ebegin);
-        const uint32_t o1 = p0 + (uint32_t)(__ldg(a.off + t.vbegin + r + 1) - t.ebegin);
-        s.off[r] = (uint16_t)o0;
-        if (r + 1 == nrows) s.off[nrows] = (uint16_t)o1;
-        if (o1 > o0) {
-          // lanes whose span starts inside this row; the first row with
-          // edges also takes the lanes that start in the empty slots before
-          // it (p0 reaches into the second lane's span)
-          for (uint32_t k = o0 == p0 ? 0u : (o0 + kPullPer - 1) / kPullPer; k * kPullPer < o1; k++)
-            s.row[k] = (uint16_t)r;
-        }
-      }
-    }
+    if (!t.split) tile_rows(a, t, p0, s.rows);
     double acc = 0.0;
     {
       float x[kPullVec][4];
@@ -248,22 +276,17 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
       } else {
 #pragma unroll
         for (int k = 0; k < kPullVec; k++)
-          s.x[pull_slot(32u * k + lane)] = make_float4(x[k][0], x[k][1], x[k][2], x[k][3]);
+          s.x[slot_word(32u * k + lane)] = make_float4(x[k][0], x[k][1], x[k][2], x[k][3]);
       }
     }
     const PrTile c = t;
-    const PullSpan cs = sp;
-    if (--left == 0) {
-      ti = __shfl_sync(kFull, drawn, 0);
-      left = a.draw;
-    } else {
-      ti++;
-    }
+    const TileSpan cs = sp;
+    ti = take_tile(a, draw, ti);
     if (c.split) {
       // the rest of a long row's part
       for (uint32_t first = 32 * kPullVec; first < cs.nvec; first += 32 * kPullVec) {
         float x[kPullVec][4];
-        pull_ids(cs, first, q);
+        tile_words<4>(cs, first, q);
         pull_gather(a, first, p0, p1, q, x);
 #pragma unroll
         for (int k = 0; k < kPullVec; k++)
@@ -272,8 +295,8 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
     }
     if (ti < a.ntiles) {
       t = a.tiles[ti];
-      sp = pull_span(a, t);
-      pull_ids(sp, 0, q);
+      sp = tile_span<4>(a, t);
+      tile_words<4>(sp, 0, q);
     }
     if (c.split) {
       acc = warp_sum(acc);
@@ -296,14 +319,14 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
       continue;
     }
     __syncwarp();  // contributions and row table are in place
-    const uint32_t b0 = kPullPer * lane;  // this lane's span [b0, b0 + kPullPer)
+    const uint32_t b0 = kPer * lane;  // this lane's span [b0, b0 + kPer)
     uint32_t key = 0x10000u + lane;       // row whose open part this lane holds; else its own
     if (p1 > p0 && b0 < p1) {
-      uint32_t r = s.row[lane], end = s.off[r + 1];
-      bool open = s.off[r] < b0;  // the row began in an earlier span
+      uint32_t r = s.rows.row[lane], end = s.rows.off[r + 1];
+      bool open = s.rows.off[r] < b0;  // the row began in an earlier span
 #pragma unroll
       for (int k = 0; k < kPullVec; k++) {
-        const float4 f = s.x[pull_slot(kPullVec * lane + k)];
+        const float4 f = s.x[slot_word(kPullVec * lane + k)];
         const float x[4] = {f.x, f.y, f.z, f.w};
 #pragma unroll
         for (int j = 0; j < 4; j++) {
@@ -313,13 +336,13 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
             acc = 0.0;
             open = false;
             do r++;
-            while (s.off[r + 1] <= p);
-            end = s.off[r + 1];
+            while (s.rows.off[r + 1] <= p);
+            end = s.rows.off[r + 1];
           }
           acc += (double)x[j];
         }
       }
-      if (open || end > b0 + kPullPer) key = r;
+      if (open || end > b0 + kPer) key = r;
       else s.sum[r] = acc;
     }
     __syncwarp();
@@ -345,8 +368,118 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
   if (threadIdx.x == 0 && dsum != 0.0) atomicAdd(a.dang + a.it + 1, dsum);
 }
 
+// Push scatter, one tile per warp (the tiles and slots of the pull): every
+// slot's source contribution is laid out by the lane whose span holds the
+// slot, then the ids, striped over the lanes, add it to their sums, kPer
+// FP64 reductions in flight per lane while the next tile's ids load.  Two
+// CTAs per SM fill the reduction units; more only queue behind them (RMAT
+// 4.2 M vertices, resident: 1 CTA 574 us per iteration, 2 438, 3 438, 4 485).
+//
+// Per iteration against pr_push_cta_kernel: 3,000 vertices 21.4 -> 13.0 us,
+// 262 K (4.1 M edges) 56.2 -> 50.8; with half the edges over the link, 262 K
+// 359 -> 336 us and 3 M vertices (35 M edges) 1,562 -> 1,520 us (loads of
+// whole lines: 46.9 -> 48.2 GB/s over the link).  Resident from 12 M edges up it
+// is 438 us against 460 or 136 against 129, depending on where the hubs' sums
+// fall: one L2 slice at 94% of its requests bounds both, so those keep the
+// CTA kernel.
+constexpr int kPushCtas = 2;
+constexpr uint64_t kPushWarpEdges = 8ull << 20;
+struct PushWarp {
+  float4 x[kSlots / 4];  // source contribution of each slot
+  float c[kRows];        // and of each row
+  WarpRows rows;
+};
+
 template <int ESZ>
-__global__ void __launch_bounds__(kPrThreads) pr_push_kernel(PrArgs a) {
+__global__ void __launch_bounds__(kPrThreads, 4) pr_push_kernel(PrArgs a) {
+  constexpr int EPW = 16 / ESZ;      // edges per 16-byte word
+  constexpr int NV = kPer / EPW;     // words per lane
+  __shared__ PushWarp s_warp[kPrWarps];
+  PushWarp &s = s_warp[threadIdx.x >> 5];
+  const unsigned lane = lane_id();
+  TileDraw draw;
+  uint32_t ti = first_tile(a, draw);
+  PrTile t{};
+  TileSpan sp{};
+  uint4 qn[NV];
+  if (ti < a.ntiles) {
+    t = a.tiles[ti];
+    sp = tile_span<ESZ>(a, t);
+    tile_words<ESZ>(sp, 0, qn);
+  }
+  while (ti < a.ntiles) {
+    ask_tile(a, draw);
+    const PrTile c = t;
+    const TileSpan cs = sp;
+    const uint32_t p0 = cs.p0, p1 = p0 + (uint32_t)(c.eend - c.ebegin);
+    float cv = 0.f;  // split tiles: the row's contribution
+    if (c.split) {
+      cv = __ldg(a.cur + c.vbegin);
+    } else {
+      for (uint32_t r = lane; r < c.vend - c.vbegin; r += 32) s.c[r] = __ldg(a.cur + c.vbegin + r);
+      tile_rows(a, c, p0, s.rows);
+      __syncwarp();
+      const uint32_t b0 = kPer * lane;
+      if (p1 > p0 && b0 < p1) {
+        uint32_t r = s.rows.row[lane], end = s.rows.off[r + 1];
+        float f = s.c[r];
+#pragma unroll
+        for (int k = 0; k < kPer / 4; k++) {
+          float x[4];
+#pragma unroll
+          for (int j = 0; j < 4; j++) {
+            const uint32_t p = b0 + 4u * k + j;
+            if (p >= end && p < p1) {
+              do r++;
+              while (s.rows.off[r + 1] <= p);
+              end = s.rows.off[r + 1];
+              f = s.c[r];
+            }
+            x[j] = f;
+          }
+          s.x[slot_word((kPer / 4) * lane + k)] = make_float4(x[0], x[1], x[2], x[3]);
+        }
+      }
+      __syncwarp();
+    }
+    uint4 q[NV];
+#pragma unroll
+    for (int k = 0; k < NV; k++) q[k] = qn[k];
+    ti = take_tile(a, draw, ti);
+    if (ti < a.ntiles) {
+      t = a.tiles[ti];
+      sp = tile_span<ESZ>(a, t);
+      tile_words<ESZ>(sp, 0, qn);
+    }
+    for (uint32_t first = 0;;) {
+#pragma unroll
+      for (int k = 0; k < NV; k++) {
+        const uint32_t v = first + 32u * k + lane, p = EPW * v;
+        const uint32_t e[4] = {q[k].x, q[k].y, q[k].z, q[k].w};
+        float f[4] = {cv, cv, cv, cv};
+        if (!c.split) {
+          // EPW slots of the 16-byte word that holds slot p
+          const float *w = reinterpret_cast<const float *>(&s.x[slot_word(p / 4)]) + (p & 3u);
+#pragma unroll
+          for (int j = 0; j < EPW; j++) f[j] = w[j];
+        }
+#pragma unroll
+        for (int j = 0; j < EPW; j++)
+          if (p + j >= p0 && p + j < p1)
+            atomicAdd(a.sum + (ESZ == 4 ? edge_dst(e[j], a.wshift) : e[2 * j]), (double)f[j]);
+      }
+      first += 32 * NV;
+      if (first >= cs.nvec) break;  // only split tiles go on
+      tile_words<ESZ>(cs, first, q);
+    }
+    __syncwarp();
+  }
+}
+
+// Push with a tile per CTA, staged in shared memory: resident graphs of at
+// least kPushWarpEdges edges.
+template <int ESZ>
+__global__ void __launch_bounds__(kPrThreads) pr_push_cta_kernel(PrArgs a) {
   __shared__ __align__(16) uint32_t s_e[kStageEdges * (ESZ / 4) + 16];
   __shared__ uint32_t s_tile;
   const unsigned lane = lane_id(), warp = threadIdx.x >> 5;
@@ -453,7 +586,7 @@ __global__ void pr_widen(const float *rank, uint64_t nv, uint64_t half, double *
 //         inactive (pr_kernels.cu:846-860, frontier cleared each round at
 //         src/pr/pr.cu:1067-1077).
 // Rounds run until no vertex is active.  The gather/scatter kernels reuse
-// the tiles of the fixed-iteration kernels and skip tiles without an active
+// tiles sized for a CTA and skip tiles without an active
 // vertex, so converged regions cost one flag read per vertex.  Pull sums are
 // warp-segmented (fixed order) with atomics only across the parts of a split
 // vertex; push adds with FP64 atomics like the reference.
@@ -764,12 +897,14 @@ static thv_status ensure_pr_state(thv_graph *g, bool push, uint32_t iters, bool 
 }
 
 template <int ESZ>
-static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, uint32_t iters,
+static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, PrTileKind kind, uint32_t iters,
                              cudaStream_t st, uint32_t &launches) {
   PrState *p = g->ps;
   int bpsm = 0;
-  if (push)
-    THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_push_kernel<ESZ>, kPrThreads, 0));
+  if (push && kind == kWarpTiles)
+    bpsm = kPushCtas;
+  else if (push)
+    THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_push_cta_kernel<ESZ>, kPrThreads, 0));
   else
     THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_pull_kernel, kPrThreads, 0));
   const int grid = std::max(1, bpsm) * g->num_sms;
@@ -783,7 +918,8 @@ static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, uint32_t iters,
     a.cur = p->d_c[it & 1];
     a.nxt = p->d_c[(it + 1) & 1];
     if (push) {
-      pr_push_kernel<ESZ><<<grid, kPrThreads, 0, st>>>(a);
+      if (kind == kWarpTiles) pr_push_kernel<ESZ><<<grid, kPrThreads, 0, st>>>(a);
+      else pr_push_cta_kernel<ESZ><<<grid, kPrThreads, 0, st>>>(a);
       pr_push_update<<<ugrid, kPrThreads, 0, st>>>(a);
       launches += 2;
     } else {
@@ -888,7 +1024,8 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   const uint32_t iters = o && o->pr_iters ? o->pr_iters : 20u;
   const double damping = o && o->pr_damping > 0 ? o->pr_damping : 0.85;
   THV_TRY(ensure_plan(g));
-  const PrTileKind kind = push ? kCtaTiles : kWarpTiles;
+  const PrTileKind kind =
+      push && g->plan.host_edge_bytes == 0 && g->ne >= kPushWarpEdges ? kCtaTiles : kWarpTiles;
   THV_TRY(build_tiles(g, kind));
   const PrTiles &tiles = g->plan.tiles[kind];
   THV_TRY(ensure_pr_state(g, push, iters, false, tiles));
@@ -924,8 +1061,8 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   pr_init<<<ugrid, kPrThreads, 0, st>>>(a, p->d_c[0]);
   THV_CUDA(cudaGetLastError());
   launches++;
-  thv_status s = g->esz == 8 ? pr_iterate<8>(g, a, push, iters, st, launches)
-                             : pr_iterate<4>(g, a, push, iters, st, launches);
+  thv_status s = g->esz == 8 ? pr_iterate<8>(g, a, push, kind, iters, st, launches)
+                             : pr_iterate<4>(g, a, push, kind, iters, st, launches);
   if (s != THV_OK) return s;
   THV_CUDA(cudaEventRecord(p->ev1, st));
   THV_CUDA(cudaStreamSynchronize(st));

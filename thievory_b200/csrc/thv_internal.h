@@ -52,16 +52,16 @@ struct __align__(16) PrTile {
   uint32_t split;  // 0, or 1 + index of the split vertex
 };
 
-// Tile sets, built lazily per plan: sized for one CTA (push, and the
-// reference-semantics kernels) or for one warp (pull).
+// Tile sets, built lazily per plan: sized for one CTA (push on
+// large resident graphs, the reference-semantics kernels) or for one warp.
 enum PrTileKind { kCtaTiles = 0, kWarpTiles = 1 };
 struct PrTileShape {
   uint64_t edges, verts;  // bounds of a tile
   uint64_t split_deg;     // a vertex above this is cut into split tiles
   uint64_t part_edges;    // edges of one split tile
 };
-// Pull keeps a tile's edges in 512 slots counted from a 128-byte line, so
-// up to 31 of them lie before its first edge; its split tiles take up to
+// A warp keeps its tile's edges in 512 slots counted from a 128-byte line,
+// so up to 31 of them lie before the first edge; split tiles take up to
 // 2,048 such slots.
 constexpr PrTileShape kTileShape[2] = {{4096, 2048, 1024, 4096}, {480, 128, 480, 2016}};
 struct PrTiles {
