@@ -306,6 +306,56 @@ __device__ __forceinline__ void ms_sssp_item(const MsArgs &a, uint32_t ring, uin
   }
 }
 
+// Splits the pending sources f (lane = vertex v0 + lane, vertices wd) by
+// their distance: take holds those below thr, keep the rest, kmin the least
+// kept distance.  Each half-warp reads one vertex's whole row, 16 bytes per
+// lane (the layout of ms_sssp_item), kSplitPer rows in flight per half-warp;
+// ballots turn the lanes' comparisons into the vertex's mask.  (One lane per
+// vertex, reading its pending sources' words one by one, fetched a 32-byte
+// sector per word: eight times the row.)
+constexpr int kSplitPer = 4;
+__device__ __forceinline__ void ms_split_pending(const MsArgs &a, uint32_t v0, uint32_t wd,
+                                                 unsigned long long f, uint32_t thr,
+                                                 unsigned long long &take, unsigned long long &keep,
+                                                 uint32_t &kmin) {
+  const unsigned lane = lane_id(), hl = lane & 15u, half = lane >> 4;
+  for (uint32_t m = wd; m;) {
+    int own[kSplitPer][2];  // the two vertices of each step (-1: none)
+    uint4 d[kSplitPer];
+    unsigned long long fv[kSplitPer];
+#pragma unroll
+    for (int k = 0; k < kSplitPer; k++) {
+#pragma unroll
+      for (int h = 0; h < 2; h++) {
+        own[k][h] = __ffs(m) - 1;
+        m &= m - 1;
+      }
+      const int i = half ? own[k][1] : own[k][0];
+      fv[k] = shfl64(f, i < 0 ? 0 : i);
+      if (i < 0) fv[k] = 0;
+      d[k] = i >= 0 ? __ldcg(reinterpret_cast<const uint4 *>(a.dist + (size_t)(v0 + i) * kMsWidth) + hl)
+                    : make_uint4(0, 0, 0, 0);
+    }
+#pragma unroll
+    for (int k = 0; k < kSplitPer; k++) {
+      const uint32_t dd[4] = {d[k].x, d[k].y, d[k].z, d[k].w};
+      unsigned long long lo = 0, hi = 0;
+#pragma unroll
+      for (int i = 0; i < 4; i++) {
+        const bool pend = (fv[k] >> (hl + 16u * i)) & 1ull;
+        const bool in = pend && dd[i] < thr;
+        if (pend && !in) kmin = min(kmin, dd[i]);
+        const unsigned b = __ballot_sync(kFull, in);
+        lo |= (unsigned long long)(b & 0xFFFFu) << (16 * i);
+        hi |= (unsigned long long)(b >> 16) << (16 * i);
+      }
+      if ((int)lane == own[k][0]) take = lo;
+      if ((int)lane == own[k][1]) take = hi;
+    }
+  }
+  keep = f & ~take;
+}
+
 // masks with at most this many sources relax lane-per-edge instead
 constexpr int kSparseMask = 4;
 // BFS groups of small vertices: edges per lane per step (8 spills at 64
@@ -366,9 +416,8 @@ __device__ __forceinline__ void ms_chunk(const MsArgs &a, uint32_t ring, const W
 
 // Up to gsize queued vertices per warp (q, qmask: the small or the medium
 // bucket's queue): lanes share their concatenated adjacency, so a vertex
-// gets about 32 / gsize lanes.  GS = 32 fixes gsize at compile time (the
-// two-bucket kernels); GS = 0 takes it from the argument.
-template <int OP, int ESZ, int GS>
+// gets about 32 / gsize lanes.
+template <int OP, int ESZ>
 __device__ __forceinline__ void ms_group(const MsArgs &a, uint32_t ring, const WorkItem *q,
                                          const unsigned long long *qmask, unsigned long long first,
                                          unsigned long long n_items, unsigned gsize,
@@ -377,7 +426,7 @@ __device__ __forceinline__ void ms_group(const MsArgs &a, uint32_t ring, const W
   const unsigned long long idx = first + lane;
   WorkItem it{0, 0, 0};
   unsigned long long f = 0;
-  if ((GS == 32 || lane < gsize) && idx < n_items) {
+  if (lane < gsize && idx < n_items) {
     it = q[idx];
     f = qmask[idx];
   }
@@ -442,6 +491,10 @@ __device__ __forceinline__ void ms_group(const MsArgs &a, uint32_t ring, const W
   }
 }
 
+// Tasks per warp an iteration should have for its dynamic draw to even out
+// (a group of 32 dense SSSP items is a serial chain of up to 2,000 edges).
+constexpr unsigned kTasksPerWarp = 4;
+
 // GS = 32: two degree buckets (small groups of 32 vertices per warp, chunks
 // above), the launch for the default and most tuned configurations; GS = 0:
 // three buckets with the groups' sizes from the arguments.
@@ -473,6 +526,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
     width = a.r_width;
   }
   bool yielded = false;
+  unsigned wpw = 32;
+  while (wpw > 1 && a.ngroups * (32u / wpw) < nwarps) wpw >>= 1;
   for (;; ++iter) {
     // live groups return here, between iterations: every block has passed
     // the previous iteration's last barrier, and the counter slot of this
@@ -502,11 +557,19 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
       c->minkept[nslot] = 0xFFFFFFFFu;
     }
     // ---------------------------------------------------------- compaction
+    // A warp takes wpw bitmap words at a time: 32 on large graphs, fewer
+    // while there are not enough words for every warp (with 32 words each,
+    // 147 of 4,736 warps held all of a 150,000-vertex graph's vertices, and
+    // the rest of the GPU waited for them at the barrier).  With the row
+    // reads of ms_split_pending and the smaller tasks below, one group of 64
+    // sources took, before and after (RMAT, edge factor 16): SSSP 3,000
+    // vertices 3,026 and 520 us, 150,000 4,587 and 1,642, 2.1 M 11,686 and
+    // 10,537; BFS 3,000 524 and 174, 262 K 745 and 566, 4.2 M 6,616 and 6,465.
     unsigned long long my_edges = 0, my_hbm = 0, my_link = 0, my_pairs = 0, my_keep = 0;
     uint32_t my_min = 0xFFFFFFFFu;
-    for (unsigned g = gwarp; g < a.ngroups; g += nwarps) {
-      const unsigned wbase = g * 32u;
-      const uint32_t word = ldcg(a.bm + wbase + lane);
+    for (unsigned g = gwarp; g < a.ngroups * (32u / wpw); g += nwarps) {
+      const unsigned wbase = g * wpw;
+      const uint32_t word = lane < wpw ? ldcg(a.bm + wbase + lane) : 0u;
       unsigned nz = __ballot_sync(kFull, word != 0);
       if (OP == MS_SSSP) {
         const uint32_t wm = word ? ldcg(a.wmin + wbase + lane) : 0xFFFFFFFFu;
@@ -524,35 +587,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
         const bool act = (wd >> lane) & 1u;
         unsigned long long take = 0, keep = 0;
         uint32_t kmin = 0xFFFFFFFFu;
-        if (act) {
-          const unsigned long long f = ldcg(a.front + v);
-          if (OP == MS_BFS) {
-            take = f;
-          } else {
-            // the pending sources' distances, eight loads in flight
-            const uint32_t *dv = a.dist + (size_t)v * kMsWidth;
-            unsigned long long r = f;
-            while (r) {
-              int s[8];
-              uint32_t d[8];
-#pragma unroll
-              for (int k = 0; k < 8; k++) {
-                s[k] = r ? __ffsll((long long)r) - 1 : -1;
-                r &= r - 1;
-              }
-#pragma unroll
-              for (int k = 0; k < 8; k++) d[k] = s[k] >= 0 ? ldcg(dv + row_pos((uint32_t)s[k])) : 0u;
-#pragma unroll
-              for (int k = 0; k < 8; k++) {
-                if (s[k] < 0) continue;
-                if (d[k] < thr) take |= 1ull << s[k];
-                else kmin = min(kmin, d[k]);
-              }
-            }
-            keep = f & ~take;
-          }
-          a.front[v] = keep;
-        }
+        const unsigned long long f = act ? ldcg(a.front + v) : 0ull;
+        if (OP == MS_BFS) take = f;
+        else ms_split_pending(a, (wbase + j) * 32u, wd, f, thr, take, keep, kmin);
+        if (act) a.front[v] = keep;
         const unsigned km = __ballot_sync(kFull, keep != 0);
         if (OP == MS_SSSP) {
           const uint32_t wk = warp_min(kmin);
@@ -667,18 +705,31 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
     }
     // ----------------------------------------------------------- expansion
     const uint32_t lvl1 = level + 1;
-    const unsigned gsmall = GS ? GS : a.gsmall;
+    // Small groups shrink, and chunks split into parts of whole 32-edge
+    // runs, while an iteration has too few tasks to even out over the warps.
+    // A dense SSSP item is relaxed on its own whatever its group, so SSSP
+    // groups go down to one vertex.
+    unsigned gsmall = GS ? GS : a.gsmall;
+    while (gsmall > (OP == MS_SSSP ? 1u : 4u) && nb + ns / gsmall < kTasksPerWarp * nwarps) gsmall >>= 1;
     const unsigned long long nmt = GS ? 0ull : (nm + a.gmid - 1) / a.gmid;
-    const unsigned long long ntask = nb + nmt + (ns + gsmall - 1) / gsmall;
+    const unsigned long long nrest = nmt + (ns + gsmall - 1) / gsmall;
+    const unsigned parts =
+        nb && nb + nrest < nwarps ? (unsigned)min(8ull, max(1ull, (nwarps - nrest) / nb)) : 1u;
+    const unsigned long long nbt = nb * parts, ntask = nbt + nrest;
     for (unsigned long long t = gwarp; t < ntask;) {
-      if (t < nb) {
-        ms_chunk<OP, ESZ>(a, ring, a.qb[t], a.qbm[t], lvl1);
+      if (t < nbt) {
+        WorkItem it = a.qb[t / parts];
+        const uint32_t per = ((it.cnt + parts - 1) / parts + 31u) & ~31u;
+        const uint32_t lo = min(it.cnt, (uint32_t)(t % parts) * per);
+        it.eaddr += (uint64_t)lo * ESZ;
+        it.cnt = min(it.cnt - lo, per);
+        if (it.cnt) ms_chunk<OP, ESZ>(a, ring, it, a.qbm[t / parts], lvl1);
       } else {
         // one inlined copy of the group code serves both grouped buckets
-        const bool md = GS == 0 && t < nb + nmt;
-        ms_group<OP, ESZ, GS>(a, ring, md ? a.qm : a.qs, md ? a.qmm : a.qsm,
-                              md ? (t - nb) * a.gmid : (t - nb - nmt) * gsmall, md ? nm : ns,
-                              md ? a.gmid : gsmall, lvl1);
+        const bool md = GS == 0 && t < nbt + nmt;
+        ms_group<OP, ESZ>(a, ring, md ? a.qm : a.qs, md ? a.qmm : a.qsm,
+                          md ? (t - nbt) * a.gmid : (t - nbt - nmt) * gsmall, md ? nm : ns,
+                          md ? a.gmid : gsmall, lvl1);
       }
       unsigned long long nt = 0;
       if (lane == 0) nt = nwarps + atomicAdd(&c->wc[slot], 1ull);
