@@ -32,3 +32,15 @@ def test_rows_equal_single_runs(T, O, n, k):
         got, _, _ = g.batch_run("bfs", srcs)
         for i in check:
             assert np.array_equal(got[i], O.bfs(c, int(srcs[i])))
+
+
+@pytest.mark.parametrize("wmax", [1, 64, 65, 1 << 20, (1 << 32) - 1])
+def test_default_window_follows_the_weights(T, O, wmax):
+    c = O.rmat(12, 8)
+    rng = np.random.default_rng(wmax % 1000)
+    w = O.CSR(c.off, c.adj, rng.integers(1, wmax + 1, c.ne).astype(np.uint32))
+    srcs = O.sources(c, 16).astype(np.uint32)
+    with T.Graph.from_arrays(w.off, w.wcsr_edges(), "wcsr") as g:
+        got, _, _ = g.batch_run("sssp", srcs)
+    for i in range(0, 16, 5):
+        assert np.array_equal(got[i], O.sssp(w, int(srcs[i])))

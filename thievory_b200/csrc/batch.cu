@@ -38,7 +38,19 @@ enum { MS_BFS = 0, MS_SSSP = 1 };
 constexpr uint32_t kMsWidth = 64;       // sources per group (mask bits)
 constexpr uint32_t kMaxBfsLevel = 254;  // u8 level bytes hold level + 1
 constexpr uint32_t kMsGrowth = 1;       // SSSP window width factor per advance
-constexpr uint32_t kMsDelta = 256;      // SSSP window width shared by a group
+// SSSP window width shared by a group: four times the largest weight, so
+// that the sources' waves, offset against each other by a few edges, still
+// expand a vertex in the same iteration and share its list.  At least the
+// 256 that weights up to 64 were measured with, at most 2^22 (a live group's
+// window stays clear of the distance headroom its joins keep).
+// 64 sources, before (256 whatever the weights) and after: RMAT of 150 K
+// vertices, weights to 100,000: 66.6 ms in 2,216 iterations and 2.9 in 24;
+// uniform, 400 K: 131 and 5.9; weights to 255, RMAT of 1 M: 8.3 and 7.6.
+// One, 16 times the weight: 3.7 and 2.9 ms; 5.4 and 5.9; 8.3 and 7.6.
+constexpr uint32_t kMsDeltaMin = 256, kMsDeltaMax = 1u << 22;
+static uint32_t ms_delta(const thv_graph *g) {
+  return (uint32_t)std::min<uint64_t>(kMsDeltaMax, std::max<uint64_t>(kMsDeltaMin, 4ull * g->wmax));
+}
 // SSSP: steps (two edges, one 16-byte row piece per lane each) whose rows
 // are in flight at once, staged through a per-warp shared-memory ring by
 // asynchronous copies (64 KiB per 512-thread block; 12 and 16 measured
@@ -1489,7 +1501,7 @@ thv_status run_batch_rows(thv_graph *g, thv_algo algo, const uint32_t *sources,
   // share its adjacency read (small windows make each source re-read it).
   // RMAT-26, 256 sources, weights 1..64: width 16 -> 36.6 q/s, 64 -> 74.8,
   // 128 -> 99.3, 256 -> 100.1, unbounded -> 100.1.
-  a.delta = o && o->sssp_delta ? o->sssp_delta : kMsDelta;
+  a.delta = o && o->sssp_delta ? o->sssp_delta : ms_delta(g);
   a.growth = o && o->sssp_growth ? o->sssp_growth : kMsGrowth;
 
   thv_stats local{};
@@ -1666,7 +1678,7 @@ static thv_status live_launch_any(thv_graph *g, MsArgs &a, cudaStream_t st, uint
 
 static MsArgs live_args(thv_graph *g, const LiveGroup *lg, uint32_t timeout_ms) {
   MsArgs a = ms_args(g, g->bs, timeout_ms);
-  a.delta = kMsDelta;
+  a.delta = ms_delta(g);
   a.growth = kMsGrowth;
   apply_config(a, MsConfig{lg->small, lg->chunk, lg->threads, lg->mid, lg->gsmall, lg->gmid});
   return a;
@@ -1728,8 +1740,8 @@ thv_status live_add(thv_graph *g, LiveGroup *lg, uint32_t k, const uint32_t *sou
     lg->gmid = cfg.gmid;
     lg->iter = 0;
     lg->level = 1;
-    lg->width = kMsDelta;
-    lg->thr = (uint32_t)std::min<uint64_t>(1ull + kMsDelta, 0xFFFFFFFFull);
+    lg->width = ms_delta(g);
+    lg->thr = (uint32_t)std::min<uint64_t>(1ull + ms_delta(g), 0xFFFFFFFFull);
     lg->active = 0;
   }
   THV_TRY(live_state(g, lg));

@@ -179,6 +179,7 @@ thv_status set_packing(thv_graph *g, bool on) {
       wmax = std::max(wmax, e[2 * i + 1]);
     }
     if (!ne) wmin = wmax = 0;
+    g->wmax = wmax;
     const uint32_t ib = bit_width(g->nv ? (uint32_t)(g->nv - 1) : 0u);
     const uint32_t wb = bit_width(wmax - wmin);
     if (wb >= 32 || ib + wb > 32) return THV_OK;  // does not fit: keep pairs

@@ -146,6 +146,7 @@ struct thv_graph {
   // packed weighted edges: 4 bytes = dst << wshift | (w - wbase)
   bool packed = false;
   uint32_t wshift = 0, wbase = 0;
+  uint32_t wmax = 0;  // largest edge weight
   int device = 0;
   // host
   std::vector<uint64_t> off;      // nv+1
