@@ -66,7 +66,7 @@ __host__ __device__ __forceinline__ uint32_t row_pos(uint32_t s) {
 
 struct MsCtrl {
   GridBar bar;
-  unsigned err, iters;
+  unsigned iters, pad0;
   unsigned long long cnt_small[3], cnt_big[3], remaining[3], wc[3];
   unsigned minkept[3], pad;
   unsigned long long edges, hbm_bytes, link_bytes, pairs;
@@ -556,7 +556,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
       break;
     }
     if (iter >= a.max_iters || (OP == MS_BFS && level > kMaxBfsLevel)) {
-      if (leader) atomicCAS(&c->err, 0u, OP == MS_BFS && level > kMaxBfsLevel ? kDevErrDepth : kDevErrIters);
+      if (leader) atomicCAS(&c->bar.err, 0u, OP == MS_BFS && level > kMaxBfsLevel ? kDevErrDepth : kDevErrIters);
       break;
     }
     const unsigned slot = iter % 3, nslot = (iter + 1) % 3;
@@ -643,7 +643,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
               a.qs[pos] = WorkItem{eaddr, v, deg};
               a.qsm[pos] = take;
             } else {
-              atomicCAS(&c->err, 0u, kDevErrQueue);
+              atomicCAS(&c->bar.err, 0u, kDevErrQueue);
             }
           }
         }
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
               a.qm[pos] = WorkItem{eaddr, v, deg};
               a.qmm[pos] = take;
             } else {
-              atomicCAS(&c->err, 0u, kDevErrQueue);
+              atomicCAS(&c->bar.err, 0u, kDevErrQueue);
             }
           }
         }
@@ -679,7 +679,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
                 a.qb[pos] = WorkItem{eaddr + (unsigned long long)lo * ESZ, v, min(a.chunk, deg - lo)};
                 a.qbm[pos] = take;
               } else {
-                atomicCAS(&c->err, 0u, kDevErrQueue);
+                atomicCAS(&c->bar.err, 0u, kDevErrQueue);
               }
             }
           }
@@ -704,7 +704,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
         if (my_min != 0xFFFFFFFFu) atomicMin(&c->minkept[slot], my_min);
       }
     }
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
     const unsigned long long ns = ldcg(&c->cnt_small[slot]);
     const unsigned long long nb = ldcg(&c->cnt_big[slot]);
     const unsigned long long nm = GS == 0 ? ldcg(&c->cnt_mid[slot]) : 0ull;
@@ -748,7 +748,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
       t = shfl64(nt, 0);
     }
     level++;
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
   }
   if (leader) {
     c->iters = iter;
@@ -1531,10 +1531,10 @@ thv_status run_batch_rows(thv_graph *g, thv_algo algo, const uint32_t *sources,
     THV_CUDA(cudaStreamSynchronize(st));
     cudaEventElapsedTime(ms_out, b->ev0, b->ev1);
     const MsCtrl &hc = *b->h_ctrl;
-    *deep = hc.err == kDevErrDepth;
-    if (hc.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", tmo);
-    if (hc.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
-    if (hc.err && hc.err != kDevErrDepth) return fail(THV_EDEVICE, "batch device error %u", hc.err);
+    *deep = hc.bar.err == kDevErrDepth;
+    if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", tmo);
+    if (hc.bar.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
+    if (hc.bar.err && hc.bar.err != kDevErrDepth) return fail(THV_EDEVICE, "batch device error %u", hc.bar.err);
     return THV_OK;
   };
 
@@ -1805,13 +1805,13 @@ thv_status live_step(thv_graph *g, LiveGroup *lg, uint32_t iters, uint32_t timeo
                    : live_launch_any<MS_BFS>(g, a, st, lg->threads));
   THV_CUDA(cudaStreamSynchronize(st));
   const MsCtrl &hc = *b->h_ctrl;
-  if (hc.err == kDevErrDepth) {
+  if (hc.bar.err == kDevErrDepth) {
     *too_deep = true;
     return THV_OK;
   }
-  if (hc.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", timeout_ms);
-  if (hc.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
-  if (hc.err) return fail(THV_EDEVICE, "batch device error %u", hc.err);
+  if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", timeout_ms);
+  if (hc.bar.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
+  if (hc.bar.err) return fail(THV_EDEVICE, "batch device error %u", hc.bar.err);
   lg->edges = hc.edges;
   lg->hbm_bytes = hc.hbm_bytes;
   lg->link_bytes = hc.link_bytes;

@@ -109,7 +109,7 @@ __device__ __forceinline__ MinItem make_item(unsigned long long ea, uint32_t cnt
 
 struct MinCtrl {
   GridBar bar;
-  unsigned err, iters;
+  unsigned iters, pad0;
   unsigned long long cnt_small[3], cnt_big[3], remaining[3], wc[3];
   unsigned minkept[3], pad;
   unsigned long long edges, hbm_bytes, link_bytes, vertices;
@@ -616,7 +616,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
   unsigned iter = 0;
   for (;; ++iter) {
     if (iter >= a.max_iters) {
-      if (leader) atomicCAS(&c->err, 0u, kDevErrIters);
+      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
       break;
     }
     // Counter slots.  Level L compacts into slot L % 3 and counts level
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
           c->loc_mu = lmu;
         }
       }
-      if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+      if (!grid_sync(&c->bar, a.timeout_ns)) break;
       mu = ldcg(&c->loc_mu);
       iter += ldcg(&c->loc_levels) - 1u;  // the loop's ++iter completes the jump
       listed = false;
@@ -681,7 +681,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
       bfs_bottom_up(a.in_off, a.in_adj, a.off, F, N, a.val, a.nv, lval + 1u, &c->edges,
                     &c->bu_scan[slot], &c->nf[nslot], &c->mf[nslot], gwarp, nwarps);
       if (leader) c->bu_levels++;
-      if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+      if (!grid_sync(&c->bar, a.timeout_ns)) break;
       last_scan = ldcg(&c->bu_scan[slot]);
       listed = false;
     } else {
@@ -726,7 +726,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
             const unsigned long long pos = base + __popc(sm & lanemask_lt());
             if (small) {
               if (pos < a.cap_s) a.qs[pos] = make_item(eaddr, deg, v, lval);
-              else atomicCAS(&c->err, 0u, kDevErrQueue);
+              else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
             }
           }
           if (__any_sync(kFull, big)) {
@@ -743,7 +743,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
                 if (pos < a.cap_b)
                   a.qb[pos] = make_item(eaddr + (unsigned long long)lo * ESZ, min(a.chunk, deg - lo), v, lval);
                 else
-                  atomicCAS(&c->err, 0u, kDevErrQueue);
+                  atomicCAS(&c->bar.err, 0u, kDevErrQueue);
               }
             }
           }
@@ -755,7 +755,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
         atomicAdd(&c->hbm_bytes, my_hbm);
         atomicAdd(&c->link_bytes, my_link);
       }
-      if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+      if (!grid_sync(&c->bar, a.timeout_ns)) break;
       // ------------------------------------------------------- expansion
       const unsigned long long ns = ldcg(&c->cnt_small[slot]);
       const unsigned long long nb = ldcg(&c->cnt_big[slot]);
@@ -782,7 +782,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
         atomicAdd(&c->nf[nslot], nl.nf);
         atomicAdd(&c->mf[nslot], nl.mf);
       }
-      if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+      if (!grid_sync(&c->bar, a.timeout_ns)) break;
     }
     uint32_t *x = F;
     F = N;
@@ -824,7 +824,7 @@ __global__ void __launch_bounds__(kMinThreads)
   unsigned iter = 0;
   for (;; ++iter) {
     if (iter >= a.max_iters) {
-      if (leader) atomicCAS(&c->err, 0u, kDevErrIters);
+      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
       break;
     }
     const unsigned slot = iter % 3, nslot = (iter + 1) % 3;
@@ -927,7 +927,7 @@ __global__ void __launch_bounds__(kMinThreads)
           const unsigned long long pos = base + __popc(sm & lanemask_lt());
           if (small) {
             if (pos < a.cap_s) a.qs[pos] = make_item(eaddr, deg, v, vval);
-            else atomicCAS(&c->err, 0u, kDevErrQueue);
+            else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
           }
         }
         // chunks of HBM lists fill the chunk queue from the bottom, chunks
@@ -951,7 +951,7 @@ __global__ void __launch_bounds__(kMinThreads)
                 a.qb[host ? a.cap_b - 1 - pos : pos] =
                     make_item(eaddr + (unsigned long long)lo * ESZ, cn, v, vval);
               else
-                atomicCAS(&c->err, 0u, kDevErrQueue);
+                atomicCAS(&c->bar.err, 0u, kDevErrQueue);
             }
           }
         }
@@ -997,13 +997,13 @@ __global__ void __launch_bounds__(kMinThreads)
       if (my_keep) atomicAdd(&c->remaining[slot], my_keep);
       if (my_min != 0xFFFFFFFFu) atomicMin(&c->minkept[slot], my_min);
     }
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
 
     const unsigned long long ns = ldcg(&c->cnt_small[slot]);
     const unsigned long long nb = ldcg(&c->cnt_big[slot]);
     const unsigned long long nh = ldcg(&c->cnt_host[slot]);
     if (nb + nh > a.cap_b) {  // the two ends of the chunk queue met
-      if (leader) atomicCAS(&c->err, 0u, kDevErrQueue);
+      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrQueue);
       break;
     }
     if (ns + nb + nh == 0) {
@@ -1068,7 +1068,7 @@ __global__ void __launch_bounds__(kMinThreads)
         t = first + shfl64(nt, 0);
       }
     }
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
   }
   if (leader) c->iters = iter;
 }
@@ -1205,7 +1205,7 @@ __device__ __forceinline__ void q_append(const MinArgs &a, const uint32_t *vb,
   if (small) {
     const unsigned long long pos = b_s + __popc(sm & lanemask_lt());
     if (pos < a.cap_s) qs[pos] = make_item(eaddr, deg, w, wval);
-    else atomicCAS(&c->err, 0u, kDevErrQueue);
+    else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
   }
   if (big) {
     unsigned long long pos = host ? b_h + inc_h - nch : b_r + inc_r - nch;
@@ -1215,7 +1215,7 @@ __device__ __forceinline__ void q_append(const MinArgs &a, const uint32_t *vb,
         qb[host ? a.cap_b - 1 - pos : pos] =
             make_item(eaddr + (unsigned long long)lo * ESZ, min(a.chunk, deg - lo), w, wval);
       else
-        atomicCAS(&c->err, 0u, kDevErrQueue);
+        atomicCAS(&c->bar.err, 0u, kDevErrQueue);
     }
   }
 }
@@ -1509,7 +1509,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
   bool scan = true;
   for (;; ++iter, ++ph) {
     if (iter >= a.max_iters) {
-      if (leader) atomicCAS(&c->err, 0u, kDevErrIters);
+      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
       break;
     }
     const unsigned cur = ph % 3, prev = (ph + 2) % 3;
@@ -1668,10 +1668,10 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
       }
       q_flush<ESZ>(a, env, nst, true, qst);
     }
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
     const unsigned long long nbig = ldcg(&c->cnt_big[cur]), nhost = ldcg(&c->cnt_host[cur]);
     if (nbig + nhost > a.cap_b) {  // the two ends of the chunk queue met
-      if (leader) atomicCAS(&c->err, 0u, kDevErrQueue);
+      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrQueue);
       break;
     }
     const unsigned long long produced = ldcg(&c->cnt_small[cur]) + nbig + nhost;
@@ -1866,7 +1866,7 @@ __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
       const unsigned long long pos = base + __popc(sm & lanemask_lt());
       if (small) {
         if (pos < a.cap_s) a.qs[pos] = make_item(eaddr, cnt, v, v);
-        else atomicCAS(&c->err, 0u, kDevErrQueue);
+        else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
       }
     }
     if (__any_sync(kFull, big)) {
@@ -1883,7 +1883,7 @@ __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
           if (pos < a.cap_b)
             a.qb[pos] = make_item(eaddr + (unsigned long long)lo * ESZ, min(a.chunk, cnt - lo), v, v);
           else
-            atomicCAS(&c->err, 0u, kDevErrQueue);
+            atomicCAS(&c->bar.err, 0u, kDevErrQueue);
         }
       }
     }
@@ -2218,13 +2218,13 @@ thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
     stats->checksum = want_sum ? hc.checksum : 0;
     stats->bottom_up_levels = hc.bu_levels;
   }
-  if (hc.err == kDevErrBarrier)
+  if (hc.bar.err == kDevErrBarrier)
     return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", tmo);
-  if (hc.err == kDevErrIters)
+  if (hc.bar.err == kDevErrIters)
     return fail(THV_ETIMEOUT, "iteration cap %u reached", a.max_iters);
-  if (hc.err == kDevErrQueue)
+  if (hc.bar.err == kDevErrQueue)
     return fail(THV_EDEVICE, "work queue overflow");
-  if (hc.err) return fail(THV_EDEVICE, "device error %u", hc.err);
+  if (hc.bar.err) return fail(THV_EDEVICE, "device error %u", hc.bar.err);
   return THV_OK;
 }
 
@@ -2390,10 +2390,10 @@ static thv_status bfs_noalloc(const uint64_t *d_off, const uint32_t *d_adj, uint
   THV_CUDA(cudaMemcpyAsync(&hc, a.ctrl, sizeof(MinCtrl), cudaMemcpyDeviceToHost, st));
   THV_CUDA(cudaStreamSynchronize(st));
   if (iterations) *iterations = hc.iters;
-  if (hc.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait timed out");
-  if (hc.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
-  if (hc.err == kDevErrQueue) return fail(THV_EDEVICE, "work queue overflow");
-  if (hc.err) return fail(THV_EDEVICE, "device error %u", hc.err);
+  if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait timed out");
+  if (hc.bar.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
+  if (hc.bar.err == kDevErrQueue) return fail(THV_EDEVICE, "work queue overflow");
+  if (hc.bar.err) return fail(THV_EDEVICE, "device error %u", hc.bar.err);
   return THV_OK;
 }
 

@@ -80,9 +80,9 @@ extern "C" thv_status thv_link_bandwidth(int device, uint64_t bytes, double *mem
 // fault (the wait is limited by %globaltimer and always ends).
 namespace thv {
 
-__global__ void wait_timeout_probe(GridBar *bar, unsigned *err, unsigned long long timeout_ns) {
+__global__ void wait_timeout_probe(GridBar *bar, unsigned long long timeout_ns) {
   if (blockIdx.x == 0) return;
-  grid_sync(bar, err, timeout_ns);
+  grid_sync(bar, timeout_ns);
 }
 
 }  // namespace thv
@@ -92,19 +92,15 @@ extern "C" thv_status thv_debug_wait_timeout(int device, uint32_t timeout_ms) {
   try {
     if (timeout_ms == 0 || timeout_ms > 10000) return fail(THV_EINVAL, "timeout must be 1..10000 ms");
     THV_CUDA(cudaSetDevice(device));
-    struct Scratch {
-      GridBar bar;
-      unsigned err, pad;
-    };
-    Scratch *d = nullptr;
-    THV_TRY(dev_alloc((void **)&d, sizeof(Scratch), "wait probe"));
-    Scratch h{};
+    GridBar *d = nullptr;
+    THV_TRY(dev_alloc((void **)&d, sizeof(GridBar), "wait probe"));
+    GridBar h{};
     thv_status s = THV_OK;
-    if (cudaMemset(d, 0, sizeof(Scratch)) != cudaSuccess) s = fail(THV_ECUDA, "memset");
+    if (cudaMemset(d, 0, sizeof(GridBar)) != cudaSuccess) s = fail(THV_ECUDA, "memset");
     if (s == THV_OK) {
-      wait_timeout_probe<<<2, 32>>>(&d->bar, &d->err, (unsigned long long)timeout_ms * 1000000ull);
+      wait_timeout_probe<<<2, 32>>>(d, (unsigned long long)timeout_ms * 1000000ull);
       if (cudaGetLastError() != cudaSuccess || cudaDeviceSynchronize() != cudaSuccess ||
-          cudaMemcpy(&h, d, sizeof(Scratch), cudaMemcpyDeviceToHost) != cudaSuccess)
+          cudaMemcpy(&h, d, sizeof(GridBar), cudaMemcpyDeviceToHost) != cudaSuccess)
         s = fail(THV_ECUDA, "wait probe launch failed");
     }
     dev_free(d);

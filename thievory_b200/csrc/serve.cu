@@ -49,7 +49,7 @@ constexpr uint32_t kSvDeltaSssp = 256;  // shared-read sweet spot (batched sweep
 
 struct SvCtrl {
   GridBar bar;
-  unsigned err, iters;
+  unsigned iters, pad0;
   unsigned long long cnt_small[3], cnt_big[3], wc[3];
   unsigned long long taken_or[3], alive_or[3];
   unsigned thr[kSvMaxSlots], step[kSvMaxSlots];
@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kSvThreads) sv_kernel(SvArgs a) {
               a.qs[pos] = WorkItem{eaddr, v, deg};
               a.qsm[pos] = take;
             } else {
-              atomicCAS(&c->err, 0u, kDevErrQueue);
+              atomicCAS(&c->bar.err, 0u, kDevErrQueue);
             }
           }
         }
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kSvThreads) sv_kernel(SvArgs a) {
                 a.qb[pos] = WorkItem{eaddr + (unsigned long long)lo * ESZ, v, min(a.chunk, deg - lo)};
                 a.qbm[pos] = take;
               } else {
-                atomicCAS(&c->err, 0u, kDevErrQueue);
+                atomicCAS(&c->bar.err, 0u, kDevErrQueue);
               }
             }
           }
@@ -360,7 +360,7 @@ __global__ void __launch_bounds__(kSvThreads) sv_kernel(SvArgs a) {
         atomicAdd(&c->pairs, my_pairs);
       }
     }
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
     const unsigned long long taken = ldcg(&c->taken_or[slot]);
     const unsigned long long alive = ldcg(&c->alive_or[slot]);
     done = a.active & ~alive;
@@ -388,7 +388,7 @@ __global__ void __launch_bounds__(kSvThreads) sv_kernel(SvArgs a) {
       s_step[s] = st;
       s_thr[s] = (uint32_t)min((unsigned long long)s_thr[s] + st, 0xFFFFFFFFull);
     }
-    if (!grid_sync(&c->bar, &c->err, a.timeout_ns)) break;
+    if (!grid_sync(&c->bar, a.timeout_ns)) break;
     if (done) {
       ++iter;
       break;
@@ -629,8 +629,8 @@ thv_status step(thv_server *s, uint32_t max_iters, unsigned long long *done, uin
   THV_CUDA(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, sizeof(SvCtrl), cudaMemcpyDeviceToHost, s->st));
   THV_CUDA(cudaStreamSynchronize(s->st));
   const SvCtrl &hc = *s->h_ctrl;
-  if (hc.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "serving: grid barrier timeout");
-  if (hc.err) return fail(THV_EDEVICE, "serving: device error %u", hc.err);
+  if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "serving: grid barrier timeout");
+  if (hc.bar.err) return fail(THV_EDEVICE, "serving: device error %u", hc.bar.err);
   *done = hc.done_mask;
   *iters = hc.iters;
   return THV_OK;
