@@ -261,7 +261,7 @@ typedef struct thv_stats {
 } thv_stats;
 
 /* Runs algo.  out_values (host, may be NULL) receives u32[nv] or double[nv]
- * (PR).  stats may be NULL.  Synchronous. */
+ * (PR), unspecified when the call fails.  stats may be NULL.  Synchronous. */
 thv_status thv_run(thv_graph *g, thv_algo algo, const thv_run_opts *o,
                    void *out_values, thv_stats *stats);
 /* Copy the last run's values (u32[nv], or double[nv] for PR) to the host. */

@@ -1056,11 +1056,8 @@ thv_status thv_run(thv_graph *g, thv_algo algo, const thv_run_opts *o,
     case THV_ALGO_BFS:
     case THV_ALGO_CC:
     case THV_ALGO_SSSP:
-      s = run_minprop(g, algo, o, st, &local);
-      if (s == THV_OK && out_values) {
-        s = minprop_values(g, (uint32_t *)out_values, st);
-        local.d2h_bytes += g->nv * 4;
-      }
+      s = run_minprop(g, algo, o, st, &local, (uint32_t *)out_values);
+      if (s == THV_OK && out_values) local.d2h_bytes += g->nv * 4;
       break;
     case THV_ALGO_PR_PUSH:
     case THV_ALGO_PR_PULL:

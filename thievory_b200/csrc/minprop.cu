@@ -181,6 +181,15 @@ struct MinState {
   uint32_t ngroups = 0;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   bool valid = false;
+  // launch shape of the kernels run on this state: the occupancy query and
+  // the attribute cost a small graph's call several microseconds each
+  struct Shape {
+    const void *kern;
+    size_t smem;
+    int grid;
+  };
+  Shape shapes[8] = {};
+  int nshapes = 0;
 };
 
 // Position of the n-th (from 0) set bit of x; n < popc(x).
@@ -1101,6 +1110,10 @@ __global__ void minprop_init(MinArgs a, uint32_t nw_alloc) {
     // and the second frontier bitmap of direction-optimising runs
     if (OP == OP_BFS && a.wmin) a.wmin[w] = 0;
     if (OP == OP_BFS && a.bm2) a.bm2[w] = 0;
+    if (a.qbits) {  // queue mode: nothing is queued in either phase parity
+      a.qbits[w] = 0;
+      a.qbits[nw_alloc + w] = 0;
+    }
   }
   if (tid == 0) {
     MinCtrl *c = a.ctrl;
@@ -1695,11 +1708,6 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
   if (leader) c->iters = iter;
 }
 
-__global__ void minq_clear(uint32_t *qbits, uint32_t nwords) {
-  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < nwords; i += gridDim.x * blockDim.x)
-    qbits[i] = 0;
-}
-
 __global__ void values_checksum_kernel(const uint32_t *val, uint64_t nv,
                                        unsigned long long *sum) {
   __shared__ unsigned long long s_red[32];
@@ -2038,27 +2046,45 @@ void minprop_free(thv_graph *g) {
   g->ms = nullptr;
 }
 
+// Shared memory of a plan's block table (first vertices and bases), and of
+// the largest one kept there.
+static size_t block_table_bytes(size_t nb) { return nb * 8 + (nb + 1) * 4; }
+constexpr size_t kMaxTableBytes = kSmemBlocks * 8 + (kSmemBlocks + 1) * 4;
+
+// Blocks of a cooperative launch of kern with smem bytes, looked up once per
+// state and plan size.  Every caller allows the largest table, so no launch
+// on another graph ever finds a lower limit.
+static thv_status launch_grid(thv_graph *g, const void *kern, size_t smem, int *grid) {
+  MinState *ms = g->ms;
+  for (int i = 0; i < ms->nshapes; i++)
+    if (ms->shapes[i].kern == kern && ms->shapes[i].smem == smem) {
+      *grid = ms->shapes[i].grid;
+      return THV_OK;
+    }
+  THV_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxTableBytes));
+  int bpsm = 0;
+  THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, kern, kMinThreads, smem));
+  if (bpsm < 1) return fail(THV_ECUDA, "minprop kernel cannot be resident");
+  if (ms->nshapes == 8) ms->nshapes = 0;  // many re-plans: start over
+  ms->shapes[ms->nshapes++] = {kern, smem, bpsm * g->num_sms};
+  *grid = bpsm * g->num_sms;
+  return THV_OK;
+}
+
 template <int OP, int ESZ>
 static thv_status launch_minprop(thv_graph *g, MinArgs &a, cudaStream_t st,
                                  uint32_t &launches, bool scan_mode) {
   auto kern = scan_mode ? (OP == OP_BFS && a.do_alpha ? bfs_do_kernel<ESZ> : minprop_kernel<OP, ESZ>)
                         : minq_kernel<OP, ESZ>;
   const size_t nb = g->plan.blocks.size();
-  const size_t smem = nb <= kSmemBlocks ? nb * 8 + (nb + 1) * 4 : 0;
-  THV_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  int bpsm = 0;
-  THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, kern,
-                                                         kMinThreads, smem));
-  if (bpsm < 1) return fail(THV_ECUDA, "minprop kernel cannot be resident");
-  const int grid = bpsm * g->num_sms;
+  const size_t smem = nb <= kSmemBlocks ? block_table_bytes(nb) : 0;
+  int grid = 0;
+  THV_TRY(launch_grid(g, (const void *)kern, smem, &grid));
   const uint32_t nw_alloc = g->ms->ngroups * 32u;
   const int init_grid = std::max(1, std::min<int>(g->num_sms * 8,
                                 (int)((g->nv + 255) / 256)));
+  if (scan_mode || OP == OP_BFS) a.qbits = nullptr;
   minprop_init<OP><<<init_grid, 256, 0, st>>>(a, nw_alloc);
-  if (!scan_mode && OP != OP_BFS) {
-    minq_clear<<<init_grid, 256, 0, st>>>(a.qbits, a.ngroups * 64u);
-    launches++;
-  }
   THV_CUDA(cudaGetLastError());
   void *args[] = {&a};
   THV_CUDA(cudaLaunchCooperativeKernel((void *)kern, dim3(grid),
@@ -2067,8 +2093,11 @@ static thv_status launch_minprop(thv_graph *g, MinArgs &a, cudaStream_t st,
   return THV_OK;
 }
 
+// out (host, may be null) receives the values: their copy is queued behind
+// the traversal, so one wait covers both (two cost a small graph's call
+// about 10 us).  On an error its contents are unspecified.
 thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
-                       cudaStream_t st, thv_stats *stats) {
+                       cudaStream_t st, thv_stats *stats, uint32_t *out) {
   const int op = algo == THV_ALGO_BFS ? OP_BFS : algo == THV_ALGO_CC ? OP_CC : OP_SSSP;
   if (op == OP_SSSP && !g->weighted)
     return fail(THV_EINVAL, "SSSP needs edge weights (WCSR, or CSR opened "
@@ -2202,6 +2231,7 @@ thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   }
   THV_CUDA(cudaMemcpyAsync(ms->h_ctrl, ms->d_ctrl, sizeof(MinCtrl),
                            cudaMemcpyDeviceToHost, st));
+  if (out) THV_CUDA(cudaMemcpyAsync(out, ms->d_val, g->nv * 4, cudaMemcpyDeviceToHost, st));
   THV_CUDA(cudaStreamSynchronize(st));
   const MinCtrl &hc = *ms->h_ctrl;
   g->last_algo = algo;
@@ -2376,10 +2406,8 @@ static thv_status bfs_noalloc(const uint64_t *d_off, const uint32_t *d_adj, uint
   THV_CUDA(cudaGetLastError());
   auto kern = minprop_kernel<OP_BFS, 4>;
   const size_t smem = 1 * 8 + 2 * 4;
-  // thv_run sets this kernel's dynamic shared memory limit per plan (down
-  // to 0 for large block tables); this launch needs its own
   THV_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)smem));
+                                (int)kMaxTableBytes));
   int bpsm = 0;
   THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, kern, kMinThreads, smem));
   if (bpsm < 1) return fail(THV_ECUDA, "BFS kernel cannot be resident");

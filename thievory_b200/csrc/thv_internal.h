@@ -193,7 +193,7 @@ thv_status build_tiles(thv_graph *g, PrTileKind kind);
 void plan_free(thv_graph *g);
 
 thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
-                       cudaStream_t st, thv_stats *stats);
+                       cudaStream_t st, thv_stats *stats, uint32_t *out = nullptr);
 thv_status minprop_values(thv_graph *g, uint32_t *out, cudaStream_t st);
 const uint32_t *minprop_device_values(thv_graph *g);
 void minprop_free(thv_graph *g);
