@@ -1734,17 +1734,27 @@ __global__ void values_checksum_kernel(const uint32_t *val, uint64_t nv,
 //
 // On a symmetric graph the min-label fixed point is the smallest id of each
 // connected component, which union-find reaches without reading most of the
-// adjacency (the sampling scheme of Afforest, Sutton et al., IPDPS'18):
-//   1. every vertex unions with its first kUfSample neighbours;
-//   2. flatten; c = the component of the highest-degree vertex;
-//   3. every vertex outside c unions with the rest of its list; vertices in
-//      c skip theirs -- an edge with both ends in c changes nothing, and an
-//      edge with one end outside c is read from that end (its reverse is in
-//      the other end's list);
+// adjacency (the sampling scheme of Afforest, Sutton et al., IPDPS'18), the
+// more so when the largest component is grown as a bitmap first:
+//   1. G = the highest-degree vertex (hub) and its neighbours, then, in one
+//      or two sweeps, every vertex outside G with one of its first kUfSample
+//      neighbours in G (bit tests, no atomics on labels; skipped when the
+//      hub's list is too short to seed it, kUfHubShare).  G's members take
+//      G's least id as their parent;
+//   2. every vertex outside G unions with its first kUfSample neighbours;
+//   3. flatten; every vertex outside the hub's component unions with the
+//      rest of its list; vertices in it skip theirs -- an edge with both
+//      ends inside changes nothing, and an edge with one end outside is read
+//      from that end (its reverse is in the other end's list);
 //   4. flatten.
 // Roots are hooked larger-under-smaller with a CAS, so a parent id never
 // exceeds its child's and each root is its component's minimum id; finds
 // shortcut the path as they climb.
+//
+// Without G, step 2 builds the large component out of millions of small
+// trees, climbing and hooking each (RMAT 4 M vertices, 62 M edges, 60% of
+// them on the host: 409 of 548 us; with it the whole run takes 330).  RMAT 1
+// M: 276 -> 116 us, 20,000: 69 -> 45, 16 M: 1,595 -> 1,044.
 
 __device__ __forceinline__ uint32_t uf_find(uint32_t *p, uint32_t x) {
   uint32_t cur = ldcg(p + x);
@@ -1771,11 +1781,18 @@ __device__ __forceinline__ void uf_union(uint32_t *p, uint32_t u, uint32_t w) {
 }
 
 constexpr uint32_t kUfSample = 2;
+// The hub's neighbours seed G when they are at least one vertex in this many
+// (its sweeps then find most of the component; from a few neighbours of a
+// uniform graph they would find next to nothing).
+constexpr uint64_t kUfHubShare = 256;
+// A second sweep pays below one neighbour in 64 vertices (16 M vertices,
+// share 1/99: 1,370 us with one sweep, 1,044 with two; 4 M, 1/35: 330 and
+// 331; 1 M, 1/14: 116 and 127).
+constexpr uint64_t kUfSecondSweep = 64;
 
-// Step 1: each vertex (one thread) unions with its first kUfSample
-// neighbours.  (Storing the smallest neighbour as the parent outright, with
-// no CAS, measured slower: the parent chains it builds are long, and every
-// later find climbs them.)
+// A vertex's first kUfSample neighbours.  (Storing the smallest one as its
+// parent outright, with no CAS, measured slower: the parent chains it builds
+// are long, and every later find climbs them.)
 template <int ESZ>
 __device__ __forceinline__ void uf_sample_edges(const MinArgs &a, const uint32_t *vb,
                                                 const unsigned long long *bbase, uint32_t v,
@@ -1808,37 +1825,121 @@ __device__ __forceinline__ void uf_sample_edges(const MinArgs &a, const uint32_t
   const uint32_t *vb = smem_tab ? s_vb : a.blk_vb;                                               \
   const unsigned long long *bbase = smem_tab ? s_base : (const unsigned long long *)a.blk_base;
 
+// Step 1: the hub's neighbours into G.
 template <int ESZ>
+__global__ void __launch_bounds__(256) uf_mark(MinArgs a, uint32_t hub) {
+  const uint64_t s = __ldg(a.off + hub), e = __ldg(a.off + hub + 1);
+  bool host;
+  const unsigned long long eaddr =
+      list_addr(a.lc, __ldg(a.blk_base + find_block(a.blk_vb, a.nblk, hub)), a.host_base, hub, s,
+                (uint32_t)(e - s), ESZ, &host);
+  for (uint64_t k = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; k < e - s;
+       k += (uint64_t)gridDim.x * blockDim.x) {
+    const uint32_t raw = ld_nc_u32(eaddr + k * ESZ);
+    const uint32_t w = ESZ == 4 ? edge_dst(raw, a.wshift) : raw;
+    atomicOr(a.bm + (w >> 5), 1u << (w & 31u));
+  }
+  if (blockIdx.x == 0 && threadIdx.x == 0) {
+    atomicAdd(&a.ctrl->edges, (unsigned long long)(e - s));
+    atomicAdd(host ? &a.ctrl->link_bytes : &a.ctrl->hbm_bytes, (unsigned long long)(e - s) * ESZ);
+  }
+}
+
+// Expansion statistics of the union-find kernels: lane 0 of each warp adds.
+__device__ __forceinline__ void uf_count(const MinArgs &a, unsigned long long edges,
+                                         unsigned long long hbm, unsigned long long link) {
+  edges = warp_sum(edges);
+  hbm = warp_sum(hbm);
+  link = warp_sum(link);
+  if (lane_id() == 0 && edges) {
+    atomicAdd(&a.ctrl->edges, edges);
+    atomicAdd(&a.ctrl->hbm_bytes, hbm);
+    atomicAdd(&a.ctrl->link_bytes, link);
+  }
+}
+
+// Step 1: vertices with one of their first kUfSample neighbours in G join it
+// (a warp owns 32 vertices, one word of G; bits set meanwhile by other warps
+// may or may not be seen, either is a path to the hub).  The last sweep
+// leaves G's least id in minkept[0].
+template <int ESZ>
+__global__ void __launch_bounds__(256) uf_sweep(MinArgs a, int last) {
+  UF_STAGE_BLOCKS();
+  const unsigned lane = lane_id();
+  const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const unsigned nwarps = (gridDim.x * blockDim.x) >> 5;
+  const uint32_t nwords = (a.nv + 31) / 32;
+  unsigned long long my_edges = 0, my_hbm = 0, my_link = 0;
+  uint32_t least = 0xFFFFFFFFu;
+  for (uint32_t word = gwarp; word < nwords; word += nwarps) {
+    const uint32_t v = word * 32u + lane;
+    const uint32_t g = ldcg(a.bm + word);
+    bool in = (g >> lane) & 1u;
+    if (!in && v < a.nv) {
+      uint32_t w[kUfSample], k;
+      bool host;
+      uf_sample_edges<ESZ>(a, vb, bbase, v, w, k, host);
+      if (k) {
+#pragma unroll
+        for (uint32_t j = 0; j < kUfSample; j++)
+          in |= j < k && ((ldcg(a.bm + (w[j] >> 5)) >> (w[j] & 31u)) & 1u);
+        my_edges += k;
+        if (host) my_link += (unsigned long long)k * ESZ;
+        else my_hbm += (unsigned long long)k * ESZ;
+      }
+    }
+    const uint32_t now = __ballot_sync(kFull, in);
+    if (lane == 0 && now != g) a.bm[word] = now;
+    if (now && least == 0xFFFFFFFFu) least = word * 32u + (uint32_t)__ffs(now) - 1u;
+  }
+  if (last && lane == 0 && least != 0xFFFFFFFFu) atomicMin(&a.ctrl->minkept[0], least);
+  uf_count(a, my_edges, my_hbm, my_link);
+}
+
+// Step 2: G (when GROWN) becomes a star under its least id m, everyone else
+// and m union with their first kUfSample neighbours (a neighbour in G stands
+// for m: its own parent may not be written yet).
+template <int ESZ, bool GROWN>
 __global__ void __launch_bounds__(256) uf_sample(MinArgs a) {
   UF_STAGE_BLOCKS();
   unsigned long long my_edges = 0, my_hbm = 0, my_link = 0;
+  const uint32_t m = GROWN ? ldcg(&a.ctrl->minkept[0]) : 0u;
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.nv; v += gridDim.x * blockDim.x) {
+    if (GROWN && v != m && ((__ldg(a.bm + (v >> 5)) >> (v & 31u)) & 1u)) {
+      a.val[v] = m;
+      continue;
+    }
     uint32_t w[kUfSample], k;
     bool host;
     uf_sample_edges<ESZ>(a, vb, bbase, v, w, k, host);
     if (!k) continue;
 #pragma unroll
-    for (uint32_t j = 0; j < kUfSample; j++)
-      if (j < k && w[j] != v) uf_union(a.val, v, w[j]);
+    for (uint32_t j = 0; j < kUfSample; j++) {
+      if (j >= k || w[j] == v) continue;
+      const bool in = GROWN && ((__ldg(a.bm + (w[j] >> 5)) >> (w[j] & 31u)) & 1u);
+      uf_union(a.val, v, in ? m : w[j]);
+    }
     my_edges += k;
     if (host) my_link += (unsigned long long)k * ESZ;
     else my_hbm += (unsigned long long)k * ESZ;
   }
-  my_edges = warp_sum(my_edges);
-  my_hbm = warp_sum(my_hbm);
-  my_link = warp_sum(my_link);
-  if (lane_id() == 0 && my_edges) {
-    atomicAdd(&a.ctrl->edges, my_edges);
-    atomicAdd(&a.ctrl->hbm_bytes, my_hbm);
-    atomicAdd(&a.ctrl->link_bytes, my_link);
-  }
+  uf_count(a, my_edges, my_hbm, my_link);
 }
 
-// Step 3 work items: the lists past the sample of every vertex outside the
-// component of `hub` (labels are flattened roots here).
-template <int ESZ>
+// Root of x while no hook is in flight.
+__device__ __forceinline__ uint32_t uf_root(const uint32_t *p, uint32_t x) {
+  uint32_t r = ldcg(p + x);
+  for (uint32_t n; (n = ldcg(p + r)) != r;) r = n;
+  return r;
+}
+
+// Step 3: queues the lists past the sample of every vertex outside the
+// component of `hub`.  FLATTEN: also flattens (roots do not change here; a
+// label read before or after its own flattening has the same root), else the
+// labels are flat already.
+template <int ESZ, bool FLATTEN>
 __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
-  const uint32_t skip = ldcg(a.val + hub);
+  const uint32_t skip = FLATTEN ? uf_root(a.val, hub) : ldcg(a.val + hub);
   MinCtrl *c = a.ctrl;
   const unsigned lane = lane_id();
   const unsigned gwarp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
@@ -1849,7 +1950,9 @@ __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
     const uint32_t v = word * 32u + lane;
     uint32_t cnt = 0;
     unsigned long long eaddr = 0;
-    if (v < a.nv && ldcg(a.val + v) != skip) {
+    const uint32_t root = v >= a.nv ? skip : FLATTEN ? uf_root(a.val, v) : ldcg(a.val + v);
+    if (FLATTEN && v < a.nv) a.val[v] = root;
+    if (root != skip) {
       const uint64_t s = __ldg(a.off + v), e = __ldg(a.off + v + 1);
       const uint32_t deg = (uint32_t)(e - s);
       if (deg > kUfSample) {
@@ -1896,14 +1999,7 @@ __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
       }
     }
   }
-  my_edges = warp_sum(my_edges);
-  my_hbm = warp_sum(my_hbm);
-  my_link = warp_sum(my_link);
-  if (lane == 0 && my_edges) {
-    atomicAdd(&c->edges, my_edges);
-    atomicAdd(&c->hbm_bytes, my_hbm);
-    atomicAdd(&c->link_bytes, my_link);
-  }
+  uf_count(a, my_edges, my_hbm, my_link);
 }
 
 template <int ESZ>
@@ -1958,21 +2054,19 @@ __global__ void __launch_bounds__(256) uf_unions(MinArgs a) {
 }
 
 __global__ void uf_flatten(uint32_t *p, uint32_t nv) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x) {
-    uint32_t r = ldcg(p + v);
-    while (true) {
-      const uint32_t n = ldcg(p + r);
-      if (n == r) break;
-      r = n;
-    }
-    p[v] = r;
-  }
+  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < nv; v += gridDim.x * blockDim.x)
+    p[v] = uf_root(p, v);
 }
 
-__global__ void uf_init(MinArgs a) {
-  for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < a.nv; v += gridDim.x * blockDim.x)
-    a.val[v] = v;
-  if (blockIdx.x == 0 && threadIdx.x == 0) memset(a.ctrl, 0, sizeof(MinCtrl));
+// Every vertex its own tree; G = {hub}.
+__global__ void uf_init(MinArgs a, uint32_t hub, uint32_t nw_alloc) {
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  for (uint32_t v = tid; v < a.nv; v += stride) a.val[v] = v;
+  for (uint32_t w = tid; w < nw_alloc; w += stride) a.bm[w] = w == hub >> 5 ? 1u << (hub & 31u) : 0u;
+  if (tid == 0) {
+    memset(a.ctrl, 0, sizeof(MinCtrl));
+    a.ctrl->minkept[0] = hub;
+  }
 }
 
 // ------------------------------------------------------------------ host --
@@ -2093,6 +2187,34 @@ static thv_status launch_minprop(thv_graph *g, MinArgs &a, cudaStream_t st,
   return THV_OK;
 }
 
+template <int ESZ>
+static void launch_union_find(thv_graph *g, const MinArgs &a, cudaStream_t st, uint32_t &launches) {
+  const int grid = g->num_sms * 8;
+  const uint32_t hub = g->hub_vertex();
+  const uint64_t hub_deg = g->off[hub + 1] - g->off[hub];
+  const size_t nb = g->plan.blocks.size();
+  const size_t smem = nb <= kSmemBlocks ? block_table_bytes(nb) : 0;
+  uf_init<<<grid, 256, 0, st>>>(a, hub, g->ms->ngroups * 32u);
+  if (hub_deg * kUfHubShare >= g->nv) {
+    uf_mark<ESZ><<<g->num_sms, 256, 0, st>>>(a, hub);
+    if (hub_deg * kUfSecondSweep < g->nv) {
+      uf_sweep<ESZ><<<grid, 256, smem, st>>>(a, 0);
+      launches++;
+    }
+    uf_sweep<ESZ><<<grid, 256, smem, st>>>(a, 1);
+    uf_sample<ESZ, true><<<grid, 256, smem, st>>>(a);
+    uf_items<ESZ, true><<<grid, 256, 0, st>>>(a, hub);
+  } else {
+    // deep trees: flattened on their own first, so that later climbs are short
+    uf_sample<ESZ, false><<<grid, 256, smem, st>>>(a);
+    uf_flatten<<<grid, 256, 0, st>>>(a.val, a.nv);
+    uf_items<ESZ, false><<<grid, 256, 0, st>>>(a, hub);
+  }
+  uf_unions<ESZ><<<grid, 256, 0, st>>>(a);
+  uf_flatten<<<grid, 256, 0, st>>>(a.val, a.nv);
+  launches += hub_deg * kUfHubShare >= g->nv ? 7 : 6;
+}
+
 // out (host, may be null) receives the values: their copy is queued behind
 // the traversal, so one wait covers both (two cost a small graph's call
 // about 10 us).  On an error its contents are unspecified.
@@ -2193,24 +2315,9 @@ thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   const bool union_find = op == OP_CC && g->symmetric && g->nv > 0 &&
                           !(o && (o->flags & THV_RUN_LABEL_PROPAGATION));
   if (union_find) {
-    const int grid = g->num_sms * 8;
-    const uint32_t hub = g->hub_vertex();
-    const size_t nb = g->plan.blocks.size();
-    const size_t smem = nb <= kSmemBlocks ? nb * 8 + (nb + 1) * 4 : 0;
-    uf_init<<<grid, 256, 0, st>>>(a);
-    if (g->esz == 4) uf_sample<4><<<grid, 256, smem, st>>>(a);
-    else uf_sample<8><<<grid, 256, smem, st>>>(a);
-    uf_flatten<<<grid, 256, 0, st>>>(a.val, a.nv);
-    if (g->esz == 4) {
-      uf_items<4><<<grid, 256, 0, st>>>(a, hub);
-      uf_unions<4><<<grid, 256, 0, st>>>(a);
-    } else {
-      uf_items<8><<<grid, 256, 0, st>>>(a, hub);
-      uf_unions<8><<<grid, 256, 0, st>>>(a);
-    }
-    uf_flatten<<<grid, 256, 0, st>>>(a.val, a.nv);
+    if (g->esz == 4) launch_union_find<4>(g, a, st, launches);
+    else launch_union_find<8>(g, a, st, launches);
     THV_CUDA(cudaGetLastError());
-    launches += 6;
   } else if (g->esz == 4) {
     if (op == OP_BFS) s = launch_minprop<OP_BFS, 4>(g, a, st, launches, scan_mode);
     else if (op == OP_CC) s = launch_minprop<OP_CC, 4>(g, a, st, launches, scan_mode);
