@@ -622,20 +622,21 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
   bool bottom_up = false;
   bool listed = false;  // the last level listed the vertices it found
   const unsigned long long src_deg = __ldg(a.off + a.src + 1) - __ldg(a.off + a.src);
-  unsigned iter = 0;
-  for (;; ++iter) {
+  unsigned iter = 0;  // level
+  for (unsigned ph = 0;; ++iter, ++ph) {
     if (iter >= a.max_iters) {
       if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
       break;
     }
-    // Counter slots.  Level L compacts into slot L % 3 and counts level
-    // L+1's frontier into (L + 1) % 3, which is read at the top of level
-    // L + 1.  Slot (L + 2) % 3 of those counters was last read before level
-    // L - 1's last barrier and is next written during level L + 1, so it is
-    // cleared now.  The bottom-up scan count of level L (slot L % 3) is read
-    // just after level L's last barrier, so it is cleared one level ahead
-    // instead: slot (L + 1) % 3, last read after level L - 2's barrier.
-    const unsigned slot = iter % 3, nslot = (iter + 1) % 3, zslot = (iter + 2) % 3;
+    // Counter slots, by phase: a level on the grid, or a run of levels in
+    // one CTA.  Phase P compacts into slot P % 3 and counts the next phase's
+    // frontier into (P + 1) % 3, which is read at the top of phase P + 1.
+    // Slot (P + 2) % 3 of those counters was last read before phase P - 1's
+    // last barrier and is next written during phase P + 1, so it is cleared
+    // now.  The bottom-up scan count of phase P (slot P % 3) is read just
+    // after phase P's last barrier, so it is cleared one phase ahead instead:
+    // slot (P + 1) % 3, last read after phase P - 2's barrier.
+    const unsigned slot = ph % 3, nslot = (ph + 1) % 3, zslot = (ph + 2) % 3;
     if (leader) {
       c->cnt_small[zslot] = 0;
       c->cnt_big[zslot] = 0;
@@ -663,19 +664,11 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
         if (threadIdx.x == 0) {
           atomicAdd(&c->edges, led);
           atomicAdd(&c->hbm_bytes, led * ESZ);  // every list is resident here
-          // the grid resumes at level iter + lk with clean counters and
-          // that level's frontier size and out-edges in its slot
-          for (int k = 0; k < 3; k++) {
-            c->cnt_small[k] = 0;
-            c->cnt_big[k] = 0;
-            c->wc[k] = 0;
-            c->mf[k] = 0;
-            c->nf[k] = 0;
-            c->bu_scan[k] = 0;
-            c->fl_cnt[k] = 0;
-          }
-          c->nf[(iter + lk) % 3] = lnf;
-          c->mf[(iter + lk) % 3] = lmf;
+          // the frontier that the grid resumes with, counted as any level
+          // counts the next one (other blocks may still be reading this
+          // phase's slot)
+          c->nf[nslot] = lnf;
+          c->mf[nslot] = lmf;
           c->loc_levels = lk;
           c->loc_mu = lmu;
         }
