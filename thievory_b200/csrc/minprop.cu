@@ -158,10 +158,14 @@ struct MinArgs {
   unsigned long long ne;
   uint32_t do_alpha, do_beta;
   // queue mode: one warp in link_every draws host-list chunks first (0: none)
-  uint32_t link_every, pad3;
+  uint32_t link_every;
+  // direction-optimising BFS: 1 counts a last level without out-edges among
+  // the iterations (it is never run)
+  uint32_t count_last;
   // direction-optimising BFS: lists of small frontiers (3 slots of
   // kLocalCap vertices)
   uint32_t *flist;
+  uint64_t one_block;  // minprop_init: base of a one-entry block table to write (0: none)
 };
 
 struct MinState {
@@ -463,8 +467,8 @@ __device__ __noinline__ void bfs_bottom_up(const uint64_t *in_off, const uint32_
 // `list_in` (n_in <= kLocalCap vertices, value lv); its bits are cleared
 // from F, each level relaxes its out-edges (at most kLocalCap) edge-parallel
 // over the block, found vertices (value lv + 1, ...) form the next list in
-// shared memory, and the run stops at a frontier that is empty, holds more
-// than kLocalCap out-edges, or would go bottom-up (out-edges x alpha above
+// shared memory, and the run stops at a frontier that holds no out-edges or
+// more than kLocalCap of them, or would go bottom-up (out-edges x alpha above
 // the unexplored edges).  That frontier's bits are set in F and its size and
 // out-edges returned; *levels counts the levels run, *edges their
 // out-edges, and *mu comes back with the out-edges of every frontier after
@@ -560,7 +564,7 @@ __device__ __noinline__ void bfs_local_levels(const uint64_t *off, const uint32_
     ed += total;
     run++;
     const unsigned long long m_next = m > mf_next ? m - mf_next : 0ull;
-    if (nn == 0 || mf_next > kLocalCap || mf_next * alpha > m_next) {
+    if (mf_next == 0 || mf_next > kLocalCap || mf_next * alpha > m_next) {
       // hand the frontier back to the grid as bits
       for (uint32_t i = tid; i < nn; i += nt) {
         const uint32_t w = s_fr[cur ^ 1u][i];
@@ -648,7 +652,10 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
     }
     const unsigned long long nf = iter == 0 ? 1ull : ldcg(&c->nf[slot]);
     const unsigned long long mf = iter == 0 ? src_deg : ldcg(&c->mf[slot]);
-    if (nf == 0) break;
+    if (mf == 0) {  // no out-edges (or no vertices): nothing more to find
+      if (nf) iter += a.count_last;
+      break;
+    }
     mu = mu > mf ? mu - mf : 0;
     bottom_up = bottom_up ? nf * a.do_beta >= a.nv && 2 * mf > last_scan : mf * a.do_alpha > mu;
     const uint32_t lval = iter + 1u;  // value of this level's vertices
@@ -1112,6 +1119,11 @@ __global__ void minprop_init(MinArgs a, uint32_t nw_alloc) {
     MinCtrl *c = a.ctrl;
     memset(c, 0, sizeof(MinCtrl));
     for (int s = 0; s < 3; s++) c->minkept[s] = 0xFFFFFFFFu;
+    if (a.one_block) {
+      const_cast<uint32_t *>(a.blk_vb)[0] = 0;
+      const_cast<uint32_t *>(a.blk_vb)[1] = a.nv;
+      const_cast<uint64_t *>(a.blk_base)[0] = a.one_block;
+    }
   }
 }
 
@@ -2298,6 +2310,7 @@ thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
     a.flist = ms->d_flist;
     a.do_alpha = kBfsAlpha;
     a.do_beta = kBfsBeta;
+    a.count_last = 1;
   }
 
   uint32_t launches = 0;
@@ -2393,19 +2406,22 @@ const uint32_t *minprop_device_values(thv_graph *g) {
 namespace thv {
 
 constexpr size_t kNoAllocScratchBytes = 64ull << 20;
+constexpr uint64_t kNoAllocListEdges = 8ull << 20;  // below: small levels in one CTA
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoAllocScratchBytes];
 
 // Host code may not take the array's address directly (a host-side shadow,
 // not a device address): this is the looked-up device address per device,
-// with that device's SM count.
+// with that device's SM count and launch shapes.
 static std::mutex g_noalloc_mu;
 static uintptr_t g_noalloc_addr[64];
 static int g_noalloc_sms[64];
+static int g_noalloc_grid[64][2];
 
 static size_t align256(size_t x) { return (x + 255) & ~(size_t)255; }
 
 struct NoAllocLayout {
-  size_t ctrl, table_vb, table_base, bm, qs, qb, total;
+  size_t ctrl, table_vb, table_base, bm, qs, qb, total;  // total: what every graph needs
+  size_t bm2, flist, with_lists;                         // small levels in one CTA, if they fit
   uint32_t ngroups;
   uint64_t cap_s, cap_b;
 };
@@ -2424,17 +2440,18 @@ static NoAllocLayout noalloc_layout(uint64_t nv, uint64_t ne) {
   l.qs = off;         off += align256(l.cap_s * sizeof(MinItem));
   l.qb = off;         off += align256(l.cap_b * sizeof(MinItem));
   l.total = off;
+  l.bm2 = off;        off += align256((size_t)l.ngroups * 32 * 4);
+  l.flist = off;      off += align256(3 * kLocalCap * 4);
+  l.with_lists = off;
   return l;
 }
 
-// One edge block covering the whole graph, at the caller's adjacency.
-__global__ void noalloc_table_init(uint32_t *vb, uint64_t *base, uint32_t nv, uint64_t adj) {
-  vb[0] = 0;
-  vb[1] = nv;
-  base[0] = adj;
-}
+// Dynamic shared memory of the one-entry block table.
+constexpr size_t kNoAllocSmem = 1 * 8 + 2 * 4;
 
-static thv_status noalloc_scratch_address(int dev, uintptr_t *addr, int *sms) {
+// Scratch address, SM count and cooperative grids (small levels in one CTA,
+// every level on the grid) of a device, looked up on its first call.
+static thv_status noalloc_device(int dev, uintptr_t *addr, int *sms, int (&grid)[2]) {
   if (dev < 0 || dev >= 64) return fail(THV_EUNSUPPORTED, "device %d out of range", dev);
   std::lock_guard<std::mutex> lk(g_noalloc_mu);
   if (!g_noalloc_addr[dev]) {
@@ -2444,11 +2461,19 @@ static thv_status noalloc_scratch_address(int dev, uintptr_t *addr, int *sms) {
       return fail(THV_ECUDA, "cudaGetSymbolAddress(no-alloc scratch): %s", cudaGetErrorString(e));
     int n = 0;
     THV_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
+    const void *kern[2] = {(const void *)bfs_do_kernel<4>, (const void *)minprop_kernel<OP_BFS, 4>};
+    for (int i = 0; i < 2; i++) {
+      int bpsm = 0;
+      THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, kern[i], kMinThreads, kNoAllocSmem));
+      if (bpsm < 1) return fail(THV_ECUDA, "BFS kernel cannot be resident");
+      g_noalloc_grid[dev][i] = bpsm * n;
+    }
     g_noalloc_sms[dev] = n;
     g_noalloc_addr[dev] = (uintptr_t)p;
   }
   *addr = g_noalloc_addr[dev];
   *sms = g_noalloc_sms[dev];
+  for (int i = 0; i < 2; i++) grid[i] = g_noalloc_grid[dev][i];
   return THV_OK;
 }
 
@@ -2471,8 +2496,8 @@ static thv_status bfs_noalloc(const uint64_t *d_off, const uint32_t *d_adj, uint
   int dev = 0;
   THV_CUDA(cudaGetDevice(&dev));
   uintptr_t base = 0;
-  int sms = 0;
-  THV_TRY(noalloc_scratch_address(dev, &base, &sms));
+  int sms = 0, grid[2] = {0, 0};
+  THV_TRY(noalloc_device(dev, &base, &sms, grid));
 
   MinArgs a{};
   a.val = d_values;
@@ -2498,22 +2523,28 @@ static thv_status bfs_noalloc(const uint64_t *d_off, const uint32_t *d_adj, uint
   a.chunk = kDefaultChunk;
   a.src = source;
   a.growth = kCcGrowth;
+  a.ne = ne;
+  a.one_block = (uint64_t)(uintptr_t)d_adj;  // one block over the caller's adjacency
+  // Levels of a few vertices run inside one CTA while the others wait at a
+  // single barrier, as in thv_run's resident BFS (always top-down: there is
+  // no transpose).  A call takes 175 us instead of 185 at 150,001 vertices
+  // and 2.3 M edges, 113 instead of 128 at 10,001; at 1 M vertices and 16 M
+  // edges the found vertices' degrees cost more than the small levels save
+  // (383 and 369 us), so such graphs, and those whose scratch has no room for
+  // the frontier lists and the second bitmap, run every level on the grid.
+  const bool lists = ne < kNoAllocListEdges && l.with_lists <= kNoAllocScratchBytes;
+  if (lists) {
+    a.bm2 = (uint32_t *)(base + l.bm2);
+    a.flist = (uint32_t *)(base + l.flist);
+  }
 
-  noalloc_table_init<<<1, 1, 0, st>>>((uint32_t *)a.blk_vb, (uint64_t *)a.blk_base, (uint32_t)nv,
-                                      (uint64_t)(uintptr_t)d_adj);
   const int init_grid = std::max(1, std::min<int>(sms * 8, (int)((nv + 255) / 256)));
   minprop_init<OP_BFS><<<init_grid, 256, 0, st>>>(a, l.ngroups * 32u);
   THV_CUDA(cudaGetLastError());
-  auto kern = minprop_kernel<OP_BFS, 4>;
-  const size_t smem = 1 * 8 + 2 * 4;
-  THV_CUDA(cudaFuncSetAttribute((const void *)kern, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                (int)kMaxTableBytes));
-  int bpsm = 0;
-  THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, kern, kMinThreads, smem));
-  if (bpsm < 1) return fail(THV_ECUDA, "BFS kernel cannot be resident");
+  const void *kern = lists ? (const void *)bfs_do_kernel<4> : (const void *)minprop_kernel<OP_BFS, 4>;
   void *args[] = {&a};
-  THV_CUDA(cudaLaunchCooperativeKernel((void *)kern, dim3(bpsm * sms),
-                                       dim3(kMinThreads), args, smem, st));
+  THV_CUDA(cudaLaunchCooperativeKernel(kern, dim3(grid[lists ? 0 : 1]), dim3(kMinThreads), args,
+                                       kNoAllocSmem, st));
   MinCtrl hc;  // the caller's stack: nothing allocated
   THV_CUDA(cudaMemcpyAsync(&hc, a.ctrl, sizeof(MinCtrl), cudaMemcpyDeviceToHost, st));
   THV_CUDA(cudaStreamSynchronize(st));
