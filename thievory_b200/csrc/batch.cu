@@ -518,6 +518,8 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
   uint32_t *s_vb = reinterpret_cast<uint32_t *>(s_dyn + ring_words);
   const uint32_t ring = (uint32_t)__cvta_generic_to_shared(s_dyn) +
                         ((threadIdx.x >> 5) * kMsRing * 32u + (threadIdx.x & 31u)) * 16u;
+  __shared__ BlockCounts s_c;  // items: (vertex, source) pairs; other: medium items
+  counts_clear(s_c);
   const bool smem_tab = a.nblk <= kSmemBlocks;
   if (smem_tab)
     for (uint32_t i = threadIdx.x; i <= a.nblk; i += blockDim.x) s_vb[i] = a.blk_vb[i];
@@ -691,28 +693,37 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
     my_link = warp_sum(my_link);
     my_pairs = warp_sum(my_pairs);
     if (lane == 0 && my_edges + my_pairs) {
-      atomicAdd(&c->edges, my_edges);
-      atomicAdd(&c->hbm_bytes, my_hbm);
-      atomicAdd(&c->link_bytes, my_link);
-      atomicAdd(&c->pairs, my_pairs);
+      atomicAdd(&s_c.edges, my_edges);
+      atomicAdd(&s_c.hbm, my_hbm);
+      atomicAdd(&s_c.link, my_link);
+      atomicAdd(&s_c.items, my_pairs);
     }
     if (OP == MS_SSSP) {
       my_keep = warp_sum(my_keep);
       my_min = warp_min(my_min);
-      if (lane == 0) {
-        if (my_keep) atomicAdd(&c->remaining[slot], my_keep);
-        if (my_min != 0xFFFFFFFFu) atomicMin(&c->minkept[slot], my_min);
-      }
+      if (lane == 0) counts_kept(s_c, my_keep, my_min);
     }
-    if (!grid_sync(&c->bar, a.timeout_ns)) break;
-    const unsigned long long ns = ldcg(&c->cnt_small[slot]);
-    const unsigned long long nb = ldcg(&c->cnt_big[slot]);
-    const unsigned long long nm = GS == 0 ? ldcg(&c->cnt_mid[slot]) : 0ull;
+    if (!grid_sync(
+            &c->bar, a.timeout_ns,
+            [&] {
+              if (OP == MS_SSSP) counts_pass_kept(s_c, &c->remaining[slot], &c->minkept[slot]);
+            },
+            [&] {
+              s_c.ns = ldcg(&c->cnt_small[slot]);
+              s_c.nb = ldcg(&c->cnt_big[slot]);
+              if (GS == 0) s_c.other = ldcg(&c->cnt_mid[slot]);
+              if (OP == MS_SSSP) {
+                s_c.rem = ldcg(&c->remaining[slot]);
+                s_c.mk = ldcg(&c->minkept[slot]);
+              }
+            }))
+      break;
+    const unsigned long long ns = s_c.ns, nb = s_c.nb, nm = GS == 0 ? s_c.other : 0ull;
     if (ns + nb + nm == 0) {
       if (OP == MS_BFS) break;
-      if (ldcg(&c->remaining[slot]) == 0) break;
+      if (s_c.rem == 0) break;
       width = (uint32_t)min((unsigned long long)width * a.growth, 0xFFFFFFFFull);
-      thr = (uint32_t)min((unsigned long long)ldcg(&c->minkept[slot]) + width, 0xFFFFFFFFull);
+      thr = (uint32_t)min((unsigned long long)s_c.mk + width, 0xFFFFFFFFull);
       continue;
     }
     // ----------------------------------------------------------- expansion
@@ -749,6 +760,13 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
     }
     level++;
     if (!grid_sync(&c->bar, a.timeout_ns)) break;
+  }
+  __syncthreads();
+  if (threadIdx.x == 0 && s_c.edges + s_c.items) {
+    atomicAdd(&c->edges, s_c.edges);
+    atomicAdd(&c->hbm_bytes, s_c.hbm);
+    atomicAdd(&c->link_bytes, s_c.link);
+    atomicAdd(&c->pairs, s_c.items);
   }
   if (leader) {
     c->iters = iter;

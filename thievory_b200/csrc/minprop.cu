@@ -112,7 +112,7 @@ struct MinCtrl {
   unsigned iters, pad0;
   unsigned long long cnt_small[3], cnt_big[3], remaining[3], wc[3];
   unsigned minkept[3], pad;
-  unsigned long long edges, hbm_bytes, link_bytes, vertices;
+  unsigned long long edges, hbm_bytes, link_bytes;
   unsigned long long checksum;
   // BFS: out-edges and size of each level's frontier; bottom-up levels run
   unsigned long long mf[3], nf[3], bu_scan[3];
@@ -382,14 +382,14 @@ __device__ __forceinline__ void process_group(const MinArgs &a, unsigned long lo
 // parent in this level's frontier `front`, stopping at the first.  A warp
 // owns 32 vertices (one bitmap word) at a time, so the next frontier word is
 // its ballot, stored whole into `next`.  value = level + 1 for the vertices
-// reached here; their number and out-edges go to *next_nf / *next_mf.
+// reached here; their number and out-edges go to *next_nf / *next_mf, the
+// in-edges scanned to *level_scan (the block's counters).
 // (Scalar arguments: a MinArgs reference would copy the kernel's
 // parameter block to local memory.)
 __device__ __noinline__ void bfs_bottom_up(const uint64_t *in_off, const uint32_t *in_adj,
                                            const uint64_t *off, const uint32_t *front,
                                            uint32_t *next, uint32_t *val, uint32_t nv,
-                                           uint32_t value, unsigned long long *edges,
-                                           unsigned long long *level_scan,
+                                           uint32_t value, unsigned long long *level_scan,
                                            unsigned long long *next_nf,
                                            unsigned long long *next_mf, unsigned gwarp,
                                            unsigned nwarps) {
@@ -451,10 +451,7 @@ __device__ __noinline__ void bfs_bottom_up(const uint64_t *in_off, const uint32_
   nf = warp_sum(nf);
   mf = warp_sum(mf);
   if (lane == 0) {
-    if (scanned) {
-      atomicAdd(edges, scanned);
-      atomicAdd(level_scan, scanned);
-    }
+    if (scanned) atomicAdd(level_scan, scanned);
     if (nf) {
       atomicAdd(next_nf, nf);
       atomicAdd(next_mf, mf);
@@ -585,6 +582,16 @@ __device__ __noinline__ void bfs_local_levels(const uint64_t *off, const uint32_
   *mf_out = mf_next;
 }
 
+// A block's statistics on to the control block, at its end.
+__device__ __forceinline__ void counts_flush(MinCtrl *c, const BlockCounts &b) {
+  __syncthreads();
+  if (threadIdx.x == 0 && b.edges + b.hbm + b.link) {
+    atomicAdd(&c->edges, b.edges);
+    atomicAdd(&c->hbm_bytes, b.hbm);
+    atomicAdd(&c->link_bytes, b.link);
+  }
+}
+
 // Direction-optimising BFS on a graph whose out-edges are all resident,
 // with an in-edge transpose in HBM.  The frontier is double-buffered (F:
 // this level's, N: the next one's), and each level's direction is decided
@@ -601,6 +608,11 @@ __device__ __noinline__ void bfs_local_levels(const uint64_t *off, const uint32_
 template <int ESZ>
 __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
   extern __shared__ unsigned long long s_tab[];
+  // keep / extra: size and out-edges of the frontier found by this phase;
+  // items: in-edges scanned; ns / nb: queue sizes; rem / nh: this phase's
+  // frontier; other: in-edges the last bottom-up level scanned
+  __shared__ BlockCounts s_c;
+  counts_clear(s_c);
   const bool smem_tab = a.nblk <= kSmemBlocks;
   unsigned long long *s_base = s_tab;
   uint32_t *s_vb = reinterpret_cast<uint32_t *>(s_tab + a.nblk);
@@ -650,8 +662,27 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
       c->fl_cnt[zslot] = 0;
       c->bu_scan[nslot] = 0;
     }
-    const unsigned long long nf = iter == 0 ? 1ull : ldcg(&c->nf[slot]);
-    const unsigned long long mf = iter == 0 ? src_deg : ldcg(&c->mf[slot]);
+    const unsigned long long nf = iter == 0 ? 1ull : s_c.rem;
+    const unsigned long long mf = iter == 0 ? src_deg : s_c.nh;
+    // a phase's last barrier: what the block found goes to the next phase's
+    // slot, whose totals come back
+    auto pass_found = [&] {
+      if (s_c.keep) {
+        atomicAdd(&c->nf[nslot], s_c.keep);
+        atomicAdd(&c->mf[nslot], s_c.extra);
+        s_c.keep = s_c.extra = 0;
+      }
+      if (s_c.items) {
+        atomicAdd(&c->bu_scan[slot], s_c.items);
+        s_c.edges += s_c.items;
+        s_c.items = 0;
+      }
+    };
+    auto read_found = [&] {
+      s_c.rem = ldcg(&c->nf[nslot]);
+      s_c.nh = ldcg(&c->mf[nslot]);
+      s_c.other = ldcg(&c->bu_scan[slot]);
+    };
     if (mf == 0) {  // no out-edges (or no vertices): nothing more to find
       if (nf) iter += a.count_last;
       break;
@@ -669,8 +700,8 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
                               iter == 0 ? nullptr : a.flist + slot * kLocalCap, (uint32_t)nf,
                               a.src, lval, a.do_alpha, &lmu, &lk, &led, &lnf, &lmf);
         if (threadIdx.x == 0) {
-          atomicAdd(&c->edges, led);
-          atomicAdd(&c->hbm_bytes, led * ESZ);  // every list is resident here
+          s_c.edges += led;
+          s_c.hbm += led * ESZ;  // every list is resident here
           // the frontier that the grid resumes with, counted as any level
           // counts the next one (other blocks may still be reading this
           // phase's slot)
@@ -680,21 +711,26 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
           c->loc_mu = lmu;
         }
       }
-      if (!grid_sync(&c->bar, a.timeout_ns)) break;
-      mu = ldcg(&c->loc_mu);
-      iter += ldcg(&c->loc_levels) - 1u;  // the loop's ++iter completes the jump
+      if (!grid_sync(&c->bar, a.timeout_ns, [] {}, [&] {
+            read_found();
+            s_c.ns = ldcg(&c->loc_mu);
+            s_c.nb = ldcg(&c->loc_levels);
+          }))
+        break;
+      mu = s_c.ns;
+      iter += (unsigned)s_c.nb - 1u;  // the loop's ++iter completes the jump
       listed = false;
       continue;  // F already holds the next level's frontier
     }
     if (bottom_up) {
-      bfs_bottom_up(a.in_off, a.in_adj, a.off, F, N, a.val, a.nv, lval + 1u, &c->edges,
-                    &c->bu_scan[slot], &c->nf[nslot], &c->mf[nslot], gwarp, nwarps);
+      bfs_bottom_up(a.in_off, a.in_adj, a.off, F, N, a.val, a.nv, lval + 1u, &s_c.items, &s_c.keep,
+                    &s_c.extra, gwarp, nwarps);
       if (leader) c->bu_levels++;
-      if (!grid_sync(&c->bar, a.timeout_ns)) break;
-      last_scan = ldcg(&c->bu_scan[slot]);
+      if (!grid_sync(&c->bar, a.timeout_ns, pass_found, read_found)) break;
+      last_scan = s_c.other;
       listed = false;
     } else {
-      if (leader) atomicAdd(&c->edges, mf);
+      if (leader) s_c.edges += mf;
       // ------------------------------------------------------ compaction
       unsigned long long my_hbm = 0, my_link = 0;
       for (unsigned g = gwarp / nsub; g < a.ngroups && gwarp / nsub < gstride; g += gstride) {
@@ -761,13 +797,16 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
       my_hbm = warp_sum(my_hbm);
       my_link = warp_sum(my_link);
       if (lane == 0 && my_hbm + my_link) {
-        atomicAdd(&c->hbm_bytes, my_hbm);
-        atomicAdd(&c->link_bytes, my_link);
+        atomicAdd(&s_c.hbm, my_hbm);
+        atomicAdd(&s_c.link, my_link);
       }
-      if (!grid_sync(&c->bar, a.timeout_ns)) break;
+      if (!grid_sync(&c->bar, a.timeout_ns, [] {}, [&] {
+            s_c.ns = ldcg(&c->cnt_small[slot]);
+            s_c.nb = ldcg(&c->cnt_big[slot]);
+          }))
+        break;
       // ------------------------------------------------------- expansion
-      const unsigned long long ns = ldcg(&c->cnt_small[slot]);
-      const unsigned long long nb = ldcg(&c->cnt_big[slot]);
+      const unsigned long long ns = s_c.ns, nb = s_c.nb;
       unsigned gsize = 32;
       while (gsize > 4 && nb + (ns + gsize - 1) / gsize < nwarps / 2) gsize >>= 1;
       const unsigned long long ngrp = (ns + gsize - 1) / gsize;
@@ -788,15 +827,16 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
       nl.nf = warp_sum(nl.nf);
       nl.mf = warp_sum(nl.mf);
       if (lane == 0 && nl.nf) {
-        atomicAdd(&c->nf[nslot], nl.nf);
-        atomicAdd(&c->mf[nslot], nl.mf);
+        atomicAdd(&s_c.keep, nl.nf);
+        atomicAdd(&s_c.extra, nl.mf);
       }
-      if (!grid_sync(&c->bar, a.timeout_ns)) break;
+      if (!grid_sync(&c->bar, a.timeout_ns, pass_found, read_found)) break;
     }
     uint32_t *x = F;
     F = N;
     N = x;
   }
+  counts_flush(c, s_c);
   if (leader) c->iters = iter;
 }
 
@@ -806,6 +846,8 @@ __global__ void __launch_bounds__(kMinThreads)
   // block table (first vertex, base address) in shared memory when it fits
   extern __shared__ unsigned long long s_tab[];
   __shared__ uint32_t s_word[kMinThreads / 32][64];  // compaction: taken bits, least kept value per word
+  __shared__ BlockCounts s_c;
+  counts_clear(s_c);
   const bool smem_tab = a.nblk <= kSmemBlocks;
   unsigned long long *s_base = s_tab;
   uint32_t *s_vb = reinterpret_cast<uint32_t *>(s_tab + a.nblk);
@@ -845,9 +887,6 @@ __global__ void __launch_bounds__(kMinThreads)
       c->wc[nslot] = 0;
       c->wc_host[nslot] = 0;
       c->minkept[nslot] = 0xFFFFFFFFu;
-      c->mf[nslot] = 0;
-      c->nf[nslot] = 0;
-      c->bu_scan[nslot] = 0;
     }
     // ---------------------------------------------------------- compaction
     // A warp owns 32 bitmap words (lane = word).  The pending vertices of
@@ -857,7 +896,7 @@ __global__ void __launch_bounds__(kMinThreads)
     // per-word results (taken bits, least kept value) gather in shared
     // memory and each word is rewritten once.  Queue items come out in
     // vertex order.
-    unsigned long long my_edges = 0, my_hbm = 0, my_link = 0, my_verts = 0;
+    unsigned long long my_edges = 0, my_hbm = 0, my_link = 0;
     unsigned long long my_keep = 0;
     uint32_t my_min = 0xFFFFFFFFu;
     uint32_t *s_tk = s_word[threadIdx.x >> 5], *s_km = s_tk + 32;
@@ -920,7 +959,6 @@ __global__ void __launch_bounds__(kMinThreads)
           eaddr = list_addr(a.lc, bbase[bi], a.host_base, v, s0, deg, ESZ, &host);
           if (a.blk_access) atomicAdd(a.blk_access + bi, (unsigned long long)deg * ESZ);
           my_edges += deg;
-          my_verts += 1;
           if (host) my_link += (unsigned long long)deg * ESZ;
           else my_hbm += (unsigned long long)deg * ESZ;
         }
@@ -985,45 +1023,45 @@ __global__ void __launch_bounds__(kMinThreads)
     my_edges = warp_sum(my_edges);
     my_hbm = warp_sum(my_hbm);
     my_link = warp_sum(my_link);
-    my_verts = warp_sum(my_verts);
     if (OP != OP_BFS) {
       my_min = warp_min(my_min);
       my_keep = warp_sum(my_keep);
     }
-    if (lane == 0 && my_verts) {
-      // BFS edges are counted once the level's direction is known
-      if (OP == OP_BFS) {
-        atomicAdd(&c->mf[slot], my_edges);
-        atomicAdd(&c->nf[slot], my_verts);
-      } else {
-        atomicAdd(&c->edges, my_edges);
-      }
-      atomicAdd(&c->hbm_bytes, my_hbm);
-      atomicAdd(&c->link_bytes, my_link);
-      atomicAdd(&c->vertices, my_verts);
+    if (lane == 0 && my_edges) {
+      atomicAdd(&s_c.edges, my_edges);
+      atomicAdd(&s_c.hbm, my_hbm);
+      atomicAdd(&s_c.link, my_link);
     }
-    if (OP != OP_BFS && lane == 0) {
-      if (my_keep) atomicAdd(&c->remaining[slot], my_keep);
-      if (my_min != 0xFFFFFFFFu) atomicMin(&c->minkept[slot], my_min);
-    }
-    if (!grid_sync(&c->bar, a.timeout_ns)) break;
+    if (OP != OP_BFS && lane == 0) counts_kept(s_c, my_keep, my_min);
+    if (!grid_sync(
+            &c->bar, a.timeout_ns,
+            [&] {
+              if (OP != OP_BFS) counts_pass_kept(s_c, &c->remaining[slot], &c->minkept[slot]);
+            },
+            [&] {
+              s_c.ns = ldcg(&c->cnt_small[slot]);
+              s_c.nb = ldcg(&c->cnt_big[slot]);
+              s_c.nh = ldcg(&c->cnt_host[slot]);
+              if (OP != OP_BFS) {
+                s_c.rem = ldcg(&c->remaining[slot]);
+                s_c.mk = ldcg(&c->minkept[slot]);
+              }
+            }))
+      break;
 
-    const unsigned long long ns = ldcg(&c->cnt_small[slot]);
-    const unsigned long long nb = ldcg(&c->cnt_big[slot]);
-    const unsigned long long nh = ldcg(&c->cnt_host[slot]);
+    const unsigned long long ns = s_c.ns, nb = s_c.nb, nh = s_c.nh;
     if (nb + nh > a.cap_b) {  // the two ends of the chunk queue met
       if (leader) atomicCAS(&c->bar.err, 0u, kDevErrQueue);
       break;
     }
     if (ns + nb + nh == 0) {
       if (OP == OP_BFS) break;
-      if (ldcg(&c->remaining[slot]) == 0) break;
-      const uint32_t mk = ldcg(&c->minkept[slot]);
+      if (s_c.rem == 0) break;
+      const uint32_t mk = s_c.mk;
       width = (uint32_t)min((unsigned long long)width * a.growth, 0xFFFFFFFFull);
       thr = (uint32_t)min((unsigned long long)mk + width, 0xFFFFFFFFull);
       continue;
     }
-    if (OP == OP_BFS && leader) atomicAdd(&c->edges, ldcg(&c->mf[slot]));
     // ----------------------------------------------------------- expansion
     // task ids: chunks first, then groups of 32 small vertices; each warp
     // starts on task gwarp, then draws from a shared counter (no atomic at
@@ -1079,6 +1117,7 @@ __global__ void __launch_bounds__(kMinThreads)
     }
     if (!grid_sync(&c->bar, a.timeout_ns)) break;
   }
+  counts_flush(c, s_c);
   if (leader) c->iters = iter;
 }
 
@@ -1493,6 +1532,8 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
   // staging list: fewer than 32 carried entries plus one relaxation step's
   __shared__ uint2 s_stage[kMinThreads / 32][32 * (kQRelaxMax + 1)];
   __shared__ uint32_t s_word[kMinThreads / 32][64];  // scan: taken bits, least kept value per word
+  __shared__ BlockCounts s_c;  // ns, nb, nh: what the last phase queued
+  counts_clear(s_c);
   const bool smem_tab = a.nblk <= kSmemBlocks;
   unsigned long long *s_base = s_tab;
   uint32_t *s_vb = reinterpret_cast<uint32_t *>(s_tab + a.nblk);
@@ -1621,10 +1662,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
       if (OP != OP_BFS) {
         my_keep = warp_sum(my_keep);
         my_min = warp_min(my_min);
-        if (lane == 0) {
-          if (my_keep) atomicAdd(&c->remaining[cur], my_keep);
-          if (my_min != 0xFFFFFFFFu) atomicMin(&c->minkept[cur], my_min);
-        }
+        if (lane == 0) counts_kept(s_c, my_keep, my_min);
       }
     } else {
       // --------------------------------------------------------- expansion
@@ -1636,9 +1674,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
       // the other pool.  The first task of a warp's first pool is static
       // (its index among that pool's warps), the rest come from the pool's
       // counter.
-      const unsigned long long ns = ldcg(&c->cnt_small[prev]);
-      const unsigned long long nb = ldcg(&c->cnt_big[prev]);
-      const unsigned long long nh = ldcg(&c->cnt_host[prev]);
+      const unsigned long long ns = s_c.ns, nb = s_c.nb, nh = s_c.nh;
       // With fewer tasks than warps (the small phases at a window's start
       // and end), groups shrink down to 4 vertices and each chunk is split
       // into up to 8 parts, so that more warps share the phase's edges.
@@ -1686,30 +1722,41 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
       }
       q_flush<ESZ>(a, env, nst, true, qst);
     }
-    if (!grid_sync(&c->bar, a.timeout_ns)) break;
-    const unsigned long long nbig = ldcg(&c->cnt_big[cur]), nhost = ldcg(&c->cnt_host[cur]);
-    if (nbig + nhost > a.cap_b) {  // the two ends of the chunk queue met
+    if (!grid_sync(
+            &c->bar, a.timeout_ns,
+            [&] {
+              if (OP != OP_BFS && scan) counts_pass_kept(s_c, &c->remaining[cur], &c->minkept[cur]);
+            },
+            [&] {
+              s_c.ns = ldcg(&c->cnt_small[cur]);
+              s_c.nb = ldcg(&c->cnt_big[cur]);
+              s_c.nh = ldcg(&c->cnt_host[cur]);
+              s_c.rem = ldcg(&c->remaining[cur]);
+              s_c.mk = ldcg(&c->minkept[cur]);
+            }))
+      break;
+    if (s_c.nb + s_c.nh > a.cap_b) {  // the two ends of the chunk queue met
       if (leader) atomicCAS(&c->bar.err, 0u, kDevErrQueue);
       break;
     }
-    const unsigned long long produced = ldcg(&c->cnt_small[cur]) + nbig + nhost;
-    if (produced) {
+    if (s_c.ns + s_c.nb + s_c.nh) {
       scan = false;  // expand what this phase queued
     } else if (!scan) {
       scan = true;   // near queue empty: look at the parked vertices
     } else {
-      if (OP == OP_BFS || ldcg(&c->remaining[cur]) == 0) break;
-      const uint32_t mk = ldcg(&c->minkept[cur]);
+      if (OP == OP_BFS || s_c.rem == 0) break;
+      const uint32_t mk = s_c.mk;
       width = (uint32_t)min((unsigned long long)width * a.growth, 0xFFFFFFFFull);
       thr = (uint32_t)min((unsigned long long)mk + width, 0xFFFFFFFFull);
     }
   }
   __syncwarp();
   if (lane == 0 && qst.s[0]) {
-    atomicAdd(&c->edges, qst.s[0]);
-    atomicAdd(&c->hbm_bytes, qst.s[1]);
-    atomicAdd(&c->link_bytes, qst.s[2]);
+    atomicAdd(&s_c.edges, qst.s[0]);
+    atomicAdd(&s_c.hbm, qst.s[1]);
+    atomicAdd(&s_c.link, qst.s[2]);
   }
+  counts_flush(c, s_c);
   if (leader) c->iters = iter;
 }
 
