@@ -828,72 +828,92 @@ __device__ __forceinline__ unsigned long long value_hash(uint32_t v, uint32_t va
   return x ^ (x >> 31);
 }
 
-constexpr uint32_t kExtractThreads = 256;  // ms_extract's block: 32 vertices x 64 sources per tile
-constexpr uint32_t kExtractPer = 32 * kMsWidth / kExtractThreads;
+constexpr uint32_t kExtractThreads = 256;
+// ms_extract: 16 warps of 4 sources each over tiles of 128 vertices
+constexpr uint32_t kTileVerts = 128, kTileThreads = 512;
+constexpr uint32_t kTileSources = kMsWidth / (kTileThreads / 32);
 
-// Per-source values in the single-source encoding: optional k x nv output
-// (rows per source) and a checksum per source (sum of value_hash(v, val)).
-
+// Per-source values in the single-source encoding: k x nv output (rows per
+// source) and a checksum per source (sum of value_hash(v, val)).  A tile's
+// rows come in as 16-byte pieces, the next tile's while this one is hashed
+// and written, and turn in shared memory.  Two blocks per SM: each adds its
+// 64 sums once, and with eight times as many blocks those additions, all to
+// the same few lines, took longer than the rows (262 K vertices, BFS: 107 us
+// with a byte load per value and 1,184 blocks, 31 now; SSSP, 150 K: 46 and
+// 21).
 template <int OP>
-__global__ void __launch_bounds__(kExtractThreads) ms_extract(MsArgs a, uint32_t *out,
+__global__ void __launch_bounds__(kTileThreads, 2) ms_extract(MsArgs a, uint32_t *out,
                                                              unsigned long long *sums) {
-  __shared__ unsigned long long s_sum[kMsWidth];
-  __shared__ uint32_t tile[32][kMsWidth + 1];
-  const uint32_t k = a.sources[0];
-  for (uint32_t i = threadIdx.x; i < kMsWidth; i += blockDim.x) s_sum[i] = 0;
-  // a warp always reads sources warp + 8j of a tile (j < kExtractPer), one
-  // vertex per lane: the hashes add up in registers across tiles
-  unsigned long long acc[kExtractPer];
+  constexpr uint32_t kPieces = OP == MS_BFS ? kMsWidth / 16 : kMsWidth / 4;  // 16-byte pieces of a row
+  constexpr uint32_t kLoads = kTileVerts * kPieces / kTileThreads;           // per thread and tile
+  __shared__ uint32_t tile[kMsWidth][kTileVerts + 1];
+  const uint32_t k = a.sources[0], inf = a.nv + 1u;
+  const uint32_t warp = threadIdx.x >> 5, lane = lane_id();
+  const uint4 *rows = OP == MS_BFS ? reinterpret_cast<const uint4 *>(a.lvl)
+                                   : reinterpret_cast<const uint4 *>(a.dist);
+  uint4 q[kLoads];
+  auto load = [&](uint64_t base) {
 #pragma unroll
-  for (uint32_t j = 0; j < kExtractPer; j++) acc[j] = 0;
-  __syncthreads();
-  const uint32_t inf = a.nv + 1u;
-  for (uint64_t base = (uint64_t)blockIdx.x * 32; base < a.nv; base += (uint64_t)gridDim.x * 32) {
-    for (uint32_t i = threadIdx.x; i < 32 * kMsWidth; i += kExtractThreads) {
-      const uint32_t dv = i / kMsWidth, s = i % kMsWidth;
-      const uint64_t v = base + dv;
-      uint32_t val = inf;
-      if (v < a.nv) {
-        if (OP == MS_BFS) {
-          const uint8_t l = a.lvl[v * kMsWidth + s];
-          val = l ? l : inf;
-        } else {
-          val = a.dist[v * kMsWidth + row_pos(s)];
+    for (uint32_t j = 0; j < kLoads; j++) {
+      const uint64_t i = base * kPieces + threadIdx.x + j * kTileThreads;
+      q[j] = i < (uint64_t)a.nv * kPieces ? __ldcs(rows + i) : make_uint4(0, 0, 0, 0);
+    }
+  };
+  unsigned long long acc[kTileSources] = {};
+  uint64_t base = (uint64_t)blockIdx.x * kTileVerts;
+  if (base < a.nv) load(base);
+  for (; base < a.nv; base += (uint64_t)gridDim.x * kTileVerts) {
+#pragma unroll
+    for (uint32_t j = 0; j < kLoads; j++) {
+      const uint32_t i = threadIdx.x + j * kTileThreads;
+      const uint32_t dv = i / kPieces, p = i % kPieces;
+      const uint32_t w[4] = {q[j].x, q[j].y, q[j].z, q[j].w};
+#pragma unroll
+      for (uint32_t t = 0; t < 4; t++) {
+        if (OP == MS_BFS) {  // four level bytes: sources 16p + 4t ..
+#pragma unroll
+          for (uint32_t u = 0; u < 4; u++) {
+            const uint32_t l = (w[t] >> (8 * u)) & 0xFFu;
+            tile[16 * p + 4 * t + u][dv] = l ? l : inf;
+          }
+        } else {  // source p + 16t (row_pos)
+          tile[p + 16 * t][dv] = w[t];
         }
       }
-      tile[dv][s] = val;
     }
+    const uint64_t next = base + (uint64_t)gridDim.x * kTileVerts;
+    if (next < a.nv) load(next);
     __syncthreads();
 #pragma unroll
-    for (uint32_t j = 0; j < kExtractPer; j++) {
-      const uint32_t i = threadIdx.x + j * kExtractThreads;
-      const uint32_t s = i / 32, dv = i % 32;
-      const uint64_t v = base + dv;
-      if (s < k && v < a.nv) {
-        const uint32_t val = tile[dv][s];
-        if (out) out[(uint64_t)s * a.nv + v] = val;
+    for (uint32_t j = 0; j < kTileSources; j++) {
+      const uint32_t s = warp * kTileSources + j;
+      if (s >= k) break;
+#pragma unroll
+      for (uint32_t c = 0; c < kTileVerts; c += 32) {
+        const uint64_t v = base + c + lane;
+        if (v >= a.nv) break;
+        const uint32_t val = tile[s][c + lane];
+        __stcs(out + (uint64_t)s * a.nv + v, val);
         acc[j] += value_hash((uint32_t)v, val);
       }
     }
     __syncthreads();
   }
-  if (!sums) return;
 #pragma unroll
-  for (uint32_t j = 0; j < kExtractPer; j++) {
+  for (uint32_t j = 0; j < kTileSources; j++) {
     const unsigned long long t = warp_sum(acc[j]);
-    if (lane_id() == 0 && t) atomicAdd(&s_sum[(threadIdx.x + j * kExtractThreads) / 32], t);
+    if (lane == 0 && t) atomicAdd(sums + warp * kTileSources + j, t);
   }
-  __syncthreads();
-  for (uint32_t i = threadIdx.x; i < k; i += blockDim.x)
-    if (s_sum[i]) atomicAdd(sums + i, s_sum[i]);
 }
 
 // Checksums only (no output rows): rows are read as they lie, 16 lanes per
 // row, and each lane keeps the sums of its four sources in registers (SSSP:
 // one 16-byte word = sources l, l+16, l+32, l+48; BFS: one 4-byte word =
 // level bytes of sources 4l..4l+3).
+// (Large blocks, two per SM: a block adds its 64 sums to the same few lines.)
+constexpr uint32_t kSumThreads = 1024;
 template <int OP>
-__global__ void __launch_bounds__(kExtractThreads) ms_checksum(MsArgs a, unsigned long long *sums) {
+__global__ void __launch_bounds__(kSumThreads, 2) ms_checksum(MsArgs a, unsigned long long *sums) {
   __shared__ unsigned long long s_sum[kMsWidth];
   const uint32_t k = a.sources[0];
   for (uint32_t i = threadIdx.x; i < kMsWidth; i += blockDim.x) s_sum[i] = 0;
@@ -903,7 +923,7 @@ __global__ void __launch_bounds__(kExtractThreads) ms_checksum(MsArgs a, unsigne
 #pragma unroll
   for (int i = 0; i < 4; i++) src[i] = OP == MS_BFS ? 4u * l + i : l + 16u * i;
   unsigned long long acc[4] = {0, 0, 0, 0};
-  const uint64_t rows_per = kExtractThreads / 16;
+  const uint64_t rows_per = kSumThreads / 16;
   for (uint64_t v = (uint64_t)blockIdx.x * rows_per + threadIdx.x / 16; v < a.nv;
        v += (uint64_t)gridDim.x * rows_per) {
     uint32_t val[4];
@@ -1265,11 +1285,12 @@ static thv_status enqueue_group(thv_graph *g, MsArgs &a, cudaStream_t st, bool w
   void *args[] = {&a};
   THV_CUDA(cudaLaunchCooperativeKernel((void *)kern, dim3(grid), dim3(THREADS), args, smem, st));
   THV_CUDA(cudaMemsetAsync(b->d_sums, 0, kMsWidth * 8, st));
-  const int xgrid = std::max(1, std::min<int>(g->num_sms * 8, (int)((g->nv + 31) / 32)));
+  const int xgrid =
+      std::max(1, std::min<int>(g->num_sms * 2, (int)((g->nv + kTileVerts - 1) / kTileVerts)));
   if (want_out)
-    ms_extract<OP><<<xgrid, kExtractThreads, 0, st>>>(a, b->d_out, b->d_sums);
+    ms_extract<OP><<<xgrid, kTileThreads, 0, st>>>(a, b->d_out, b->d_sums);
   else
-    ms_checksum<OP><<<g->num_sms * 8, kExtractThreads, 0, st>>>(a, b->d_sums);
+    ms_checksum<OP><<<g->num_sms * 2, kSumThreads, 0, st>>>(a, b->d_sums);
   THV_CUDA(cudaMemcpyAsync(b->h_ctrl, b->d_ctrl, sizeof(MsCtrl), cudaMemcpyDeviceToHost, st));
   THV_CUDA(cudaMemcpyAsync(b->h_sums, b->d_sums, kMsWidth * 8, cudaMemcpyDeviceToHost, st));
   THV_CUDA(cudaGetLastError());
