@@ -736,8 +736,14 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
     while (gsmall > (OP == MS_SSSP ? 1u : 4u) && nb + ns / gsmall < kTasksPerWarp * nwarps) gsmall >>= 1;
     const unsigned long long nmt = GS ? 0ull : (nm + a.gmid - 1) / a.gmid;
     const unsigned long long nrest = nmt + (ns + gsmall - 1) / gsmall;
+    // A dense SSSP chunk of 256 edges is 128 steps of a warp, some 25 us: its
+    // chunks split until there are eight tasks per warp (150 K vertices 1,620
+    // -> 1,432 us, 20 K 1,173 -> 675 and, with weights to 100,000, 912 -> 554;
+    // 2.1 M unchanged).  BFS chunks, a step of four edges per lane, only while
+    // there are warps without a task (262 K: 480 us; at eight 518).
+    const unsigned want = (OP == MS_SSSP ? 8u : 1u) * nwarps;
     const unsigned parts =
-        nb && nb + nrest < nwarps ? (unsigned)min(8ull, max(1ull, (nwarps - nrest) / nb)) : 1u;
+        nb && nb + nrest < want ? (unsigned)min(8ull, max(1ull, (want - nrest) / nb)) : 1u;
     const unsigned long long nbt = nb * parts, ntask = nbt + nrest;
     for (unsigned long long t = gwarp; t < ntask;) {
       if (t < nbt) {
