@@ -1542,7 +1542,7 @@ __device__ __forceinline__ void q_group(const MinArgs &a, const QEnv &e, const M
 }
 
 template <int OP, int ESZ>
-// Two blocks per SM: 64 registers, no spills (3 blocks spill and measured slower).
+// Two blocks per SM: 64 registers (3 blocks spill more and measured slower).
 __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
   extern __shared__ unsigned long long s_tab[];
   // staging list: fewer than 32 carried entries plus one relaxation step's
