@@ -567,7 +567,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
       break;
     }
     if (iter >= a.max_iters || (OP == MS_BFS && level > kMaxBfsLevel)) {
-      if (leader) atomicCAS(&c->bar.err, 0u, OP == MS_BFS && level > kMaxBfsLevel ? kDevErrDepth : kDevErrIters);
+      if (leader) flag_error(&c->bar, OP == MS_BFS && level > kMaxBfsLevel ? kDevErrDepth : kDevErrIters);
       break;
     }
     const unsigned slot = iter % 3, nslot = (iter + 1) % 3;
@@ -654,7 +654,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
               a.qs[pos] = WorkItem{eaddr, v, deg};
               a.qsm[pos] = take;
             } else {
-              atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+              flag_error(&c->bar, kDevErrQueue);
             }
           }
         }
@@ -671,7 +671,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
               a.qm[pos] = WorkItem{eaddr, v, deg};
               a.qmm[pos] = take;
             } else {
-              atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+              flag_error(&c->bar, kDevErrQueue);
             }
           }
         }
@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
                 a.qb[pos] = WorkItem{eaddr + (unsigned long long)lo * ESZ, v, min(a.chunk, deg - lo)};
                 a.qbm[pos] = take;
               } else {
-                atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+                flag_error(&c->bar, kDevErrQueue);
               }
             }
           }
@@ -1585,10 +1585,10 @@ thv_status run_batch_rows(thv_graph *g, thv_algo algo, const uint32_t *sources,
     THV_CUDA(cudaStreamSynchronize(st));
     cudaEventElapsedTime(ms_out, b->ev0, b->ev1);
     const MsCtrl &hc = *b->h_ctrl;
-    *deep = hc.bar.err == kDevErrDepth;
-    if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", tmo);
-    if (hc.bar.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
-    if (hc.bar.err && hc.bar.err != kDevErrDepth) return fail(THV_EDEVICE, "batch device error %u", hc.bar.err);
+    *deep = hc.bar.error() == kDevErrDepth;
+    if (hc.bar.error() == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", tmo);
+    if (hc.bar.error() == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
+    if (hc.bar.error() && hc.bar.error() != kDevErrDepth) return fail(THV_EDEVICE, "batch device error %u", hc.bar.error());
     return THV_OK;
   };
 
@@ -1859,13 +1859,13 @@ thv_status live_step(thv_graph *g, LiveGroup *lg, uint32_t iters, uint32_t timeo
                    : live_launch_any<MS_BFS>(g, a, st, lg->threads));
   THV_CUDA(cudaStreamSynchronize(st));
   const MsCtrl &hc = *b->h_ctrl;
-  if (hc.bar.err == kDevErrDepth) {
+  if (hc.bar.error() == kDevErrDepth) {
     *too_deep = true;
     return THV_OK;
   }
-  if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", timeout_ms);
-  if (hc.bar.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
-  if (hc.bar.err) return fail(THV_EDEVICE, "batch device error %u", hc.bar.err);
+  if (hc.bar.error() == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", timeout_ms);
+  if (hc.bar.error() == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
+  if (hc.bar.error()) return fail(THV_EDEVICE, "batch device error %u", hc.bar.error());
   lg->edges = hc.edges;
   lg->hbm_bytes = hc.hbm_bytes;
   lg->link_bytes = hc.link_bytes;

@@ -651,7 +651,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
   unsigned iter = 0;  // level
   for (unsigned ph = 0;; ++iter, ++ph) {
     if (iter >= a.max_iters) {
-      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
+      if (leader) flag_error(&c->bar, kDevErrIters);
       break;
     }
     // Counter slots, by phase: a level on the grid, or a run of levels in
@@ -781,7 +781,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
             const unsigned long long pos = base + __popc(sm & lanemask_lt());
             if (small) {
               if (pos < a.cap_s) a.qs[pos] = make_item(eaddr, deg, v, lval);
-              else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+              else flag_error(&c->bar, kDevErrQueue);
             }
           }
           if (__any_sync(kFull, big)) {
@@ -798,7 +798,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) bfs_do_kernel(MinArgs a) {
                 if (pos < a.cap_b)
                   a.qb[pos] = make_item(eaddr + (unsigned long long)lo * ESZ, min(a.chunk, deg - lo), v, lval);
                 else
-                  atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+                  flag_error(&c->bar, kDevErrQueue);
               }
             }
           }
@@ -885,7 +885,7 @@ __global__ void __launch_bounds__(kMinThreads)
   unsigned iter = 0;
   for (;; ++iter) {
     if (iter >= a.max_iters) {
-      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
+      if (leader) flag_error(&c->bar, kDevErrIters);
       break;
     }
     const unsigned slot = iter % 3, nslot = (iter + 1) % 3;
@@ -984,7 +984,7 @@ __global__ void __launch_bounds__(kMinThreads)
           const unsigned long long pos = base + __popc(sm & lanemask_lt());
           if (small) {
             if (pos < a.cap_s) a.qs[pos] = make_item(eaddr, deg, v, vval);
-            else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+            else flag_error(&c->bar, kDevErrQueue);
           }
         }
         // chunks of HBM lists fill the chunk queue from the bottom, chunks
@@ -1008,7 +1008,7 @@ __global__ void __launch_bounds__(kMinThreads)
                 a.qb[host ? a.cap_b - 1 - pos : pos] =
                     make_item(eaddr + (unsigned long long)lo * ESZ, cn, v, vval);
               else
-                atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+                flag_error(&c->bar, kDevErrQueue);
             }
           }
         }
@@ -1061,7 +1061,7 @@ __global__ void __launch_bounds__(kMinThreads)
 
     const unsigned long long ns = s_c.ns, nb = s_c.nb, nh = s_c.nh;
     if (nb + nh > a.cap_b) {  // the two ends of the chunk queue met
-      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+      if (leader) flag_error(&c->bar, kDevErrQueue);
       break;
     }
     if (ns + nb + nh == 0) {
@@ -1278,7 +1278,7 @@ __device__ __forceinline__ void q_append(const MinArgs &a, const uint32_t *vb,
   if (small) {
     const unsigned long long pos = b_s + __popc(sm & lanemask_lt());
     if (pos < a.cap_s) qs[pos] = make_item(eaddr, deg, w, wval);
-    else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+    else flag_error(&c->bar, kDevErrQueue);
   }
   if (big) {
     unsigned long long pos = host ? b_h + inc_h - nch : b_r + inc_r - nch;
@@ -1288,7 +1288,7 @@ __device__ __forceinline__ void q_append(const MinArgs &a, const uint32_t *vb,
         qb[host ? a.cap_b - 1 - pos : pos] =
             make_item(eaddr + (unsigned long long)lo * ESZ, min(a.chunk, deg - lo), w, wval);
       else
-        atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+        flag_error(&c->bar, kDevErrQueue);
     }
   }
 }
@@ -1584,7 +1584,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
   bool scan = true;
   for (;; ++iter, ++ph) {
     if (iter >= a.max_iters) {
-      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrIters);
+      if (leader) flag_error(&c->bar, kDevErrIters);
       break;
     }
     const unsigned cur = ph % 3, prev = (ph + 2) % 3;
@@ -1752,7 +1752,7 @@ __global__ void __launch_bounds__(kMinThreads, 2) minq_kernel(MinArgs a) {
             }))
       break;
     if (s_c.nb + s_c.nh > a.cap_b) {  // the two ends of the chunk queue met
-      if (leader) atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+      if (leader) flag_error(&c->bar, kDevErrQueue);
       break;
     }
     if (s_c.ns + s_c.nb + s_c.nh) {
@@ -2045,7 +2045,7 @@ __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
       const unsigned long long pos = base + __popc(sm & lanemask_lt());
       if (small) {
         if (pos < a.cap_s) a.qs[pos] = make_item(eaddr, cnt, v, v);
-        else atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+        else flag_error(&c->bar, kDevErrQueue);
       }
     }
     if (__any_sync(kFull, big)) {
@@ -2062,7 +2062,7 @@ __global__ void __launch_bounds__(256) uf_items(MinArgs a, uint32_t hub) {
           if (pos < a.cap_b)
             a.qb[pos] = make_item(eaddr + (unsigned long long)lo * ESZ, min(a.chunk, cnt - lo), v, v);
           else
-            atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+            flag_error(&c->bar, kDevErrQueue);
         }
       }
     }
@@ -2421,13 +2421,13 @@ thv_status run_minprop(thv_graph *g, thv_algo algo, const thv_run_opts *o,
     stats->checksum = want_sum ? hc.checksum : 0;
     stats->bottom_up_levels = hc.bu_levels;
   }
-  if (hc.bar.err == kDevErrBarrier)
+  if (hc.bar.error() == kDevErrBarrier)
     return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", tmo);
-  if (hc.bar.err == kDevErrIters)
+  if (hc.bar.error() == kDevErrIters)
     return fail(THV_ETIMEOUT, "iteration cap %u reached", a.max_iters);
-  if (hc.bar.err == kDevErrQueue)
+  if (hc.bar.error() == kDevErrQueue)
     return fail(THV_EDEVICE, "work queue overflow");
-  if (hc.bar.err) return fail(THV_EDEVICE, "device error %u", hc.bar.err);
+  if (hc.bar.error()) return fail(THV_EDEVICE, "device error %u", hc.bar.error());
   return THV_OK;
 }
 
@@ -2612,10 +2612,10 @@ static thv_status bfs_noalloc(const uint64_t *d_off, const uint32_t *d_adj, uint
   THV_CUDA(cudaMemcpyAsync(&hc, a.ctrl, sizeof(MinCtrl), cudaMemcpyDeviceToHost, st));
   THV_CUDA(cudaStreamSynchronize(st));
   if (iterations) *iterations = hc.iters;
-  if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait timed out");
-  if (hc.bar.err == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
-  if (hc.bar.err == kDevErrQueue) return fail(THV_EDEVICE, "work queue overflow");
-  if (hc.bar.err) return fail(THV_EDEVICE, "device error %u", hc.bar.err);
+  if (hc.bar.error() == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait timed out");
+  if (hc.bar.error() == kDevErrIters) return fail(THV_ETIMEOUT, "iteration cap reached");
+  if (hc.bar.error() == kDevErrQueue) return fail(THV_EDEVICE, "work queue overflow");
+  if (hc.bar.error()) return fail(THV_EDEVICE, "device error %u", hc.bar.error());
   return THV_OK;
 }
 

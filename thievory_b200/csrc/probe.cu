@@ -105,8 +105,8 @@ extern "C" thv_status thv_debug_wait_timeout(int device, uint32_t timeout_ms) {
     }
     dev_free(d);
     if (s != THV_OK) return s;
-    if (h.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", timeout_ms);
-    return fail(THV_EDEVICE, "wait probe ended without a timeout (error word %u)", h.err);
+    if (h.error() == kDevErrBarrier) return fail(THV_ETIMEOUT, "grid barrier wait exceeded %u ms", timeout_ms);
+    return fail(THV_EDEVICE, "wait probe ended without a timeout (error word %u)", h.error());
   } catch (const std::exception &e) {
     return fail(THV_ECUDA, "wait probe: %s", e.what());
   }

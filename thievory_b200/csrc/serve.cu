@@ -318,7 +318,7 @@ __global__ void __launch_bounds__(kSvThreads) sv_kernel(SvArgs a) {
               a.qs[pos] = WorkItem{eaddr, v, deg};
               a.qsm[pos] = take;
             } else {
-              atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+              flag_error(&c->bar, kDevErrQueue);
             }
           }
         }
@@ -337,7 +337,7 @@ __global__ void __launch_bounds__(kSvThreads) sv_kernel(SvArgs a) {
                 a.qb[pos] = WorkItem{eaddr + (unsigned long long)lo * ESZ, v, min(a.chunk, deg - lo)};
                 a.qbm[pos] = take;
               } else {
-                atomicCAS(&c->bar.err, 0u, kDevErrQueue);
+                flag_error(&c->bar, kDevErrQueue);
               }
             }
           }
@@ -629,8 +629,8 @@ thv_status step(thv_server *s, uint32_t max_iters, unsigned long long *done, uin
   THV_CUDA(cudaMemcpyAsync(s->h_ctrl, s->d_ctrl, sizeof(SvCtrl), cudaMemcpyDeviceToHost, s->st));
   THV_CUDA(cudaStreamSynchronize(s->st));
   const SvCtrl &hc = *s->h_ctrl;
-  if (hc.bar.err == kDevErrBarrier) return fail(THV_ETIMEOUT, "serving: grid barrier timeout");
-  if (hc.bar.err) return fail(THV_EDEVICE, "serving: device error %u", hc.bar.err);
+  if (hc.bar.error() == kDevErrBarrier) return fail(THV_ETIMEOUT, "serving: grid barrier timeout");
+  if (hc.bar.error()) return fail(THV_EDEVICE, "serving: device error %u", hc.bar.error());
   *done = hc.done_mask;
   *iters = hc.iters;
   return THV_OK;

@@ -10,7 +10,7 @@ namespace thv {
 
 constexpr unsigned kFull = 0xFFFFFFFFu;
 
-// Device error codes written into a control word (0 = ok).
+// Device error codes (0 = ok); a launch's control word holds bit code - 1.
 enum : unsigned {
   kDevOk = 0,
   kDevErrBarrier = 1,   // a grid barrier wait ran out of time
@@ -198,24 +198,36 @@ __device__ __forceinline__ unsigned long long list_addr(const ListCache &lc,
   return block_base + s0 * esz;
 }
 
-// Grid-wide barrier for a cooperative launch, with the launch's error word
-// beside it.  Every block adds 1 to `arrived`, block 0 what is missing to
-// 2^31, so the top bit flips when the last one arrives and no block resets
-// anything.  The wait is bounded by timeout_ns of %globaltimer; a block whose
-// wait runs out sets the error word, and every block that sees an error
-// leaves at once through the false return (the whole block alike).
+// Grid-wide barrier for a cooperative launch: one 64-bit word, arrivals in
+// the high half and the launch's error bits in the low one.  Every block adds
+// 1 to the arrivals, block 0 what is missing to 2^31, so their top bit flips
+// when the last one arrives and no block resets anything (the arrival scheme
+// of cooperative groups' grid barrier); what overflows leaves at the top of
+// the word, so the error bits never change by it.  The wait is bounded by
+// timeout_ns of %globaltimer; a block whose wait runs out sets its error bit,
+// and every block that sees an error leaves at once through the false return
+// (the whole block alike).
 //
-// One barrier is a release-add and the polls: an 8-byte poll reads arrivals
-// and error together.  (With a counter reset and a generation bump by the
+// The word is only ever accessed whole: PTX's memory model gives no order to
+// racing accesses that overlap in part, so a release-add on one half would
+// not synchronise with a poll of both.
+//
+// One barrier is a release-add and the polls, which read arrivals and errors
+// together.  (With a counter reset and a generation bump by the
 // last block, a 32 ns sleep between polls and the error word read by every
 // thread after the barrier, it took four dependent L2 round trips more.
 // SSSP of 700 K vertices, 46 phases: 1,113 -> 992 us; BFS of 4,999 vertices
 // 68.5 -> 59.6 us, of 1 M 146 -> 134; label propagation of 1 M, 26
 // iterations: 769 -> 668 us.)
-struct alignas(8) GridBar {
-  unsigned arrived;
-  unsigned err;
+struct GridBar {
+  unsigned long long word;
+  // code of the launch's error, the lowest of several (host, after the launch)
+  unsigned error() const { return (unsigned)__builtin_ffs((int)(unsigned)word); }
 };
+
+__device__ __forceinline__ void flag_error(GridBar *bar, unsigned code) {
+  atomicOr(&bar->word, 1ull << (code - 1u));
+}
 
 // The control block's counters sit in a few cache lines, so a phase must not
 // have every warp touch them: thread 0 of each block runs before() ahead of
@@ -236,20 +248,20 @@ __device__ __forceinline__ bool grid_sync(GridBar *bar, unsigned long long timeo
     before();
     const unsigned nblocks = gridDim.x * gridDim.y * gridDim.z;
     const unsigned add = blockIdx.x + blockIdx.y + blockIdx.z == 0 ? 0x80000000u - (nblocks - 1u) : 1u;
-    unsigned old;
+    unsigned long long old;
     // release: the block's writes, ordered before by the block barrier
-    asm volatile("atom.add.release.gpu.global.u32 %0, [%1], %2;"
-                 : "=r"(old)
-                 : "l"(&bar->arrived), "r"(add)
+    asm volatile("atom.add.release.gpu.global.u64 %0, [%1], %2;"
+                 : "=l"(old)
+                 : "l"(&bar->word), "l"((unsigned long long)add << 32)
                  : "memory");
     const unsigned long long t0 = global_ns();
     for (unsigned spins = 1;; spins++) {
       unsigned long long w;
-      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(bar) : "memory");
-      err = (unsigned)(w >> 32);
-      if (err || (((unsigned)w ^ old) & 0x80000000u)) break;
+      asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(w) : "l"(&bar->word) : "memory");
+      err = (unsigned)w;
+      if (err || (long long)(w ^ old) < 0) break;
       if ((spins & 63u) == 0 && global_ns() - t0 > timeout_ns) {
-        atomicCAS(&bar->err, 0u, kDevErrBarrier);
+        flag_error(bar, kDevErrBarrier);
         err = kDevErrBarrier;
         break;
       }
