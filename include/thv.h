@@ -135,7 +135,9 @@ thv_status thv_info(const thv_graph *g, thv_graph_info *out);
  * no effect on unweighted graphs. */
 thv_status thv_set_edge_packing(thv_graph *g, int packed);
 /* Asserts (1) or withdraws (0) that every edge u->w has its reverse w->u.
- * CC then runs as sampling union-find (THV_RUN_LABEL_PROPAGATION).
+ * CC then runs as sampling union-find (THV_RUN_LABEL_PROPAGATION).  The first
+ * assertion on a graph reads its edges once: where it does not hold, CC leaves
+ * out the shortcuts that rest on it.
  * On a graph that is not symmetric, CC with this set returns the labels of
  * its weakly connected components instead of the reference's. */
 thv_status thv_set_symmetric(thv_graph *g, int symmetric);

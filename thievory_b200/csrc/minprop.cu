@@ -1807,8 +1807,9 @@ __global__ void values_checksum_kernel(const uint32_t *val, uint64_t nv,
 //   1. G = the highest-degree vertex (hub) and its neighbours, then, in one
 //      or two sweeps, every vertex outside G with one of its first kUfSample
 //      neighbours in G (bit tests, no atomics on labels; skipped when the
-//      hub's list is too short to seed it, kUfHubShare).  G's members take
-//      G's least id as their parent;
+//      hub's list is too short to seed it, kUfHubShare, and on a graph that
+//      is marked symmetric without being so).  G's members take G's least id
+//      as their parent;
 //   2. every vertex outside G unions with its first kUfSample neighbours;
 //   3. flatten; every vertex outside the hub's component unions with the
 //      rest of its list; vertices in it skip theirs -- an edge with both
@@ -2259,8 +2260,11 @@ static void launch_union_find(thv_graph *g, const MinArgs &a, cudaStream_t st, u
   const uint64_t hub_deg = g->off[hub + 1] - g->off[hub];
   const size_t nb = g->plan.blocks.size();
   const size_t smem = nb <= kSmemBlocks ? block_table_bytes(nb) : 0;
+  // G's members leave out their own sampled edges, which only mirrored ones
+  // make up for: a graph that is marked symmetric and is not goes without G
+  const bool grown = g->mirrored == 1 && hub_deg * kUfHubShare >= g->nv;
   uf_init<<<grid, 256, 0, st>>>(a, hub, g->ms->ngroups * 32u);
-  if (hub_deg * kUfHubShare >= g->nv) {
+  if (grown) {
     uf_mark<ESZ><<<g->num_sms, 256, 0, st>>>(a, hub);
     if (hub_deg * kUfSecondSweep < g->nv) {
       uf_sweep<ESZ><<<grid, 256, smem, st>>>(a, 0);
@@ -2277,7 +2281,7 @@ static void launch_union_find(thv_graph *g, const MinArgs &a, cudaStream_t st, u
   }
   uf_unions<ESZ><<<grid, 256, 0, st>>>(a);
   uf_flatten<<<grid, 256, 0, st>>>(a.val, a.nv);
-  launches += hub_deg * kUfHubShare >= g->nv ? 7 : 6;
+  launches += grown ? 7 : 6;
 }
 
 // out (host, may be null) receives the values: their copy is queued behind

@@ -134,6 +134,7 @@ struct thv_graph {
   bool weighted = false;
   bool sorted = false;     // every adjacency list ascending by neighbour id
   bool symmetric = false;  // every u->w has w->u (asserted or by construction)
+  int mirrored = -1;       // 1: so it is, 0: it is not, -1: not looked at yet
   int64_t hub = -1;        // a vertex of maximum out-degree (lazily found)
   uint32_t hub_vertex() {
     if (hub < 0) {
@@ -182,6 +183,7 @@ namespace thv {
 
 thv_status graph_init_device(thv_graph *g);  // stream, d_off, d_outdeg
 thv_status set_packing(thv_graph *g, bool on);  // weighted graphs only
+bool edges_mirrored(const thv_graph *g);
 thv_status replan_by_access(thv_graph *g);      // THV_PLACE_ACCESS, same budget
 thv_status ensure_transpose(thv_graph *g, cudaStream_t st);  // transpose.cu
 thv_status convert_edge_list(const char *txt, const char *out_path, thv_format fmt,
