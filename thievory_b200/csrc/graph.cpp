@@ -712,6 +712,33 @@ bool edges_mirrored(const thv_graph *g) {
   return sum == 0;
 }
 
+// hub_reach is estimated from up to kReachSample evenly spaced neighbours (a
+// few random reads per thread; hubs of RMAT graphs have up to a million).
+constexpr uint64_t kReachSample = 16384;
+
+}  // namespace thv
+
+uint32_t thv_graph::hub_vertex() {
+  if (hub >= 0) return (uint32_t)hub;
+  hub = 0;
+  for (uint64_t v = 1; v < nv; v++)
+    if (off[v + 1] - off[v] > off[hub + 1] - off[hub]) hub = (int64_t)v;
+  const uint64_t deg = off[hub + 1] - off[hub];
+  const uint64_t n = std::min(deg, thv::kReachSample);
+  const uint32_t *e = (const uint32_t *)h_edges;
+  const uint32_t step = esz / 4, shift = packed ? wshift : 0;
+  uint64_t sum = 0;
+#pragma omp parallel for schedule(static) reduction(+ : sum)
+  for (int64_t i = 0; i < (int64_t)n; i++) {
+    const uint64_t w = e[step * (off[hub] + (uint64_t)i * deg / n)] >> shift;
+    sum += off[w + 1] - off[w];
+  }
+  if (n) hub_reach = (double)sum / (double)n * (double)deg / (double)ne;
+  return (uint32_t)hub;
+}
+
+namespace thv {
+
 // PageRank tiles within the bounds of kTileShape[kind], never crossing a
 // block; a vertex of more than split_deg edges is cut into parts of at most
 // part_edges edges whose partial sums are combined atomically.

@@ -1806,10 +1806,9 @@ __global__ void values_checksum_kernel(const uint32_t *val, uint64_t nv,
 // more so when the largest component is grown as a bitmap first:
 //   1. G = the highest-degree vertex (hub) and its neighbours, then, in one
 //      or two sweeps, every vertex outside G with one of its first kUfSample
-//      neighbours in G (bit tests, no atomics on labels; skipped when the
-//      hub's list is too short to seed it, kUfHubShare, and on a graph that
-//      is marked symmetric without being so).  G's members take G's least id
-//      as their parent;
+//      neighbours in G (bit tests, no atomics on labels; left out when that
+//      would not find much, kUfReach, and on a graph that is marked symmetric
+//      without being so).  G's members take G's least id as their parent;
 //   2. every vertex outside G unions with its first kUfSample neighbours;
 //   3. flatten; every vertex outside the hub's component unions with the
 //      rest of its list; vertices in it skip theirs -- an edge with both
@@ -1850,14 +1849,27 @@ __device__ __forceinline__ void uf_union(uint32_t *p, uint32_t u, uint32_t w) {
 }
 
 constexpr uint32_t kUfSample = 2;
-// The hub's neighbours seed G when they are at least one vertex in this many
-// (its sweeps then find most of the component; from a few neighbours of a
-// uniform graph they would find next to nothing).
-constexpr uint64_t kUfHubShare = 256;
-// A second sweep pays below one neighbour in 64 vertices (16 M vertices,
-// share 1/99: 1,370 us with one sweep, 1,044 with two; 4 M, 1/35: 330 and
-// 331; 1 M, 1/14: 116 and 127).
-constexpr uint64_t kUfSecondSweep = 64;
+// G pays when its sweeps find most of the component: a sampled neighbour
+// lies in G with about the share of the edges that G's members own, reach.
+// Flat graphs around one planted hub (uniform or grid, the hub's neighbours
+// 1/2 to 1/200 of the vertices) own little more than the hub's share of the
+// vertices and lose by G, up to 1.9 times with host-resident edges (1 M
+// vertices, 8 M edges, share 1/16, 40% in HBM: 773 us without, 1,299 with;
+// resident 175 and 240); what makes it pay are neighbours that are hubs
+// themselves.  Device us without G, with one sweep and with two, by reach:
+//   0.04 (power law 2.8, 100 K vertices, 40% in HBM)     87   133   156
+//   0.06 (RMAT .45/.22/.22, 1 M, resident)              850   262   258
+//   0.07 (power law 2.4, 1 M, 40% in HBM)               724   559   600
+//   0.13 (power law 2.4, 4 M, resident)               2,409   964   510
+//   0.13 (the same, 40% in HBM: the one loss found)   1,828 2,045 2,112
+//   0.39 (RMAT, 4 M, 8 M edges, 40% in HBM)             618   354   296
+//   0.46 (RMAT, 16 M)                                 1,875   849   824
+//   0.60 (RMAT, 4 M, 62 M edges, 40% in HBM)            866   335   343
+//   0.73 (RMAT, 20 K)                                    65    47    52
+// Sweeps over host-resident lists read them over the link each time, so the
+// second one needs a reach that makes its success likely.
+constexpr double kUfReach = 1.0 / 16, kUfReachOfShare = 1.5;
+constexpr double kUfOneSweep = 0.47, kUfLinkTwoSweeps = 0.25;
 
 // A vertex's first kUfSample neighbours.  (Storing the smallest one as its
 // parent outright, with no CAS, measured slower: the parent chains it builds
@@ -1984,9 +1996,8 @@ __global__ void __launch_bounds__(256) uf_sample(MinArgs a) {
     if (!k) continue;
 #pragma unroll
     for (uint32_t j = 0; j < kUfSample; j++) {
-      if (j >= k || w[j] == v) continue;
-      const bool in = GROWN && ((__ldg(a.bm + (w[j] >> 5)) >> (w[j] & 31u)) & 1u);
-      uf_union(a.val, v, in ? m : w[j]);
+      const bool in = GROWN && j < k && ((__ldg(a.bm + (w[j] >> 5)) >> (w[j] & 31u)) & 1u);
+      if (j < k && w[j] != v) uf_union(a.val, v, in ? m : w[j]);
     }
     my_edges += k;
     if (host) my_link += (unsigned long long)k * ESZ;
@@ -2257,16 +2268,17 @@ template <int ESZ>
 static void launch_union_find(thv_graph *g, const MinArgs &a, cudaStream_t st, uint32_t &launches) {
   const int grid = g->num_sms * 8;
   const uint32_t hub = g->hub_vertex();
-  const uint64_t hub_deg = g->off[hub + 1] - g->off[hub];
+  const double share = (double)(g->off[hub + 1] - g->off[hub]) / (double)g->nv, reach = g->hub_reach;
   const size_t nb = g->plan.blocks.size();
   const size_t smem = nb <= kSmemBlocks ? block_table_bytes(nb) : 0;
   // G's members leave out their own sampled edges, which only mirrored ones
   // make up for: a graph that is marked symmetric and is not goes without G
-  const bool grown = g->mirrored == 1 && hub_deg * kUfHubShare >= g->nv;
+  const bool grown = g->mirrored == 1 && reach >= kUfReach && reach > kUfReachOfShare * share;
+  const bool twice = reach < kUfOneSweep && (g->plan.host_edge_bytes == 0 || reach >= kUfLinkTwoSweeps);
   uf_init<<<grid, 256, 0, st>>>(a, hub, g->ms->ngroups * 32u);
   if (grown) {
     uf_mark<ESZ><<<g->num_sms, 256, 0, st>>>(a, hub);
-    if (hub_deg * kUfSecondSweep < g->nv) {
+    if (twice) {
       uf_sweep<ESZ><<<grid, 256, smem, st>>>(a, 0);
       launches++;
     }

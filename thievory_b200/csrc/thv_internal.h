@@ -136,14 +136,8 @@ struct thv_graph {
   bool symmetric = false;  // every u->w has w->u (asserted or by construction)
   int mirrored = -1;       // 1: so it is, 0: it is not, -1: not looked at yet
   int64_t hub = -1;        // a vertex of maximum out-degree (lazily found)
-  uint32_t hub_vertex() {
-    if (hub < 0) {
-      hub = 0;
-      for (uint64_t v = 1; v < nv; v++)
-        if (off[v + 1] - off[v] > off[hub + 1] - off[hub]) hub = (int64_t)v;
-    }
-    return (uint32_t)hub;
-  }
+  double hub_reach = 0.0;  // share of the edges that its neighbours own
+  uint32_t hub_vertex();   // finds both; at least one vertex
   // packed weighted edges: 4 bytes = dst << wshift | (w - wbase)
   bool packed = false;
   uint32_t wshift = 0, wbase = 0;
