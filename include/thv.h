@@ -280,7 +280,8 @@ typedef struct thv_batch_opts {
   uint32_t small_degree; /* expansion tuning; 0 = autotuned / default */
   uint32_t chunk_edges;  /* expansion tuning; 0 = autotuned / default */
   uint32_t sssp_delta;   /* shared near/far width for SSSP; 0 = four times
-                            the largest weight, at least 256 */
+                            the largest weight or eight times the mean one,
+                            whichever is less, within 256 .. 2^22 */
   uint32_t tune;         /* 1: without small_degree/chunk_edges, time the
                             first group under each candidate launch
                             configuration and keep the fastest (cached per

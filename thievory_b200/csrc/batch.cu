@@ -38,8 +38,9 @@ enum { MS_BFS = 0, MS_SSSP = 1 };
 constexpr uint32_t kMsWidth = 64;       // sources per group (mask bits)
 constexpr uint32_t kMaxBfsLevel = 254;  // u8 level bytes hold level + 1
 constexpr uint32_t kMsGrowth = 1;       // SSSP window width factor per advance
-// SSSP window width shared by a group: four times the largest weight, so
-// that the sources' waves, offset against each other by a few edges, still
+// SSSP window width shared by a group: four times the largest weight, or
+// eight times the mean one where that is less (the same for uniform weights),
+// so that the sources' waves, offset against each other by a few edges, still
 // expand a vertex in the same iteration and share its list.  At least the
 // 256 that weights up to 64 were measured with, at most 2^22 (a live group's
 // window stays clear of the distance headroom its joins keep).
@@ -47,9 +48,15 @@ constexpr uint32_t kMsGrowth = 1;       // SSSP window width factor per advance
 // vertices, weights to 100,000: 66.6 ms in 2,216 iterations and 2.9 in 24;
 // uniform, 400 K: 131 and 5.9; weights to 255, RMAT of 1 M: 8.3 and 7.6.
 // One, 16 times the weight: 3.7 and 2.9 ms; 5.4 and 5.9; 8.3 and 7.6.
+// By the largest weight alone, a few long edges widen the window past every
+// distance and vertices are expanded over and over.  By the largest, and the
+// mean at 8 and 16 times: grid of 300 K vertices, one weight of 10^6 among
+// weights to 64, 143 and 61 and 62 ms; Pareto weights 157, 79 and 87.  Where
+// distances are few edges long, the wider window is a little better: RMAT of
+// 150 K, Pareto weights, 0.75, 0.94 and 0.89 (all at 256: 0.94).
 constexpr uint32_t kMsDeltaMin = 256, kMsDeltaMax = 1u << 22;
 static uint32_t ms_delta(const thv_graph *g) {
-  return (uint32_t)std::min<uint64_t>(kMsDeltaMax, std::max<uint64_t>(kMsDeltaMin, 4ull * g->wmax));
+  return (uint32_t)std::min<uint64_t>(kMsDeltaMax, std::max<uint64_t>(kMsDeltaMin, 4ull * g->wtyp));
 }
 // SSSP: steps (two edges, one 16-byte row piece per lane each) whose rows
 // are in flight at once, staged through a per-warp shared-memory ring by

@@ -173,13 +173,15 @@ thv_status set_packing(thv_graph *g, bool on) {
   void *nb = nullptr;
   if (on) {
     uint32_t wmin = 0xFFFFFFFFu, wmax = 0;
-#pragma omp parallel for schedule(static) reduction(min : wmin) reduction(max : wmax)
+    uint64_t wsum = 0;  // of weights cut off at 2^22, which no window exceeds
+#pragma omp parallel for schedule(static) reduction(min : wmin) reduction(max : wmax) reduction(+ : wsum)
     for (int64_t i = 0; i < (int64_t)ne; i++) {
       wmin = std::min(wmin, e[2 * i + 1]);
       wmax = std::max(wmax, e[2 * i + 1]);
+      wsum += std::min(e[2 * i + 1], 1u << 22);
     }
     if (!ne) wmin = wmax = 0;
-    g->wmax = wmax;
+    g->wtyp = ne ? (uint32_t)std::min<uint64_t>(wmax, (2 * wsum + ne - 1) / ne) : 0;
     const uint32_t ib = bit_width(g->nv ? (uint32_t)(g->nv - 1) : 0u);
     const uint32_t wb = bit_width(wmax - wmin);
     if (wb >= 32 || ib + wb > 32) return THV_OK;  // does not fit: keep pairs

@@ -141,7 +141,7 @@ struct thv_graph {
   // packed weighted edges: 4 bytes = dst << wshift | (w - wbase)
   bool packed = false;
   uint32_t wshift = 0, wbase = 0;
-  uint32_t wmax = 0;  // largest edge weight
+  uint32_t wtyp = 0;  // twice the mean edge weight, at most the largest
   int device = 0;
   // host
   std::vector<uint64_t> off;      // nv+1
