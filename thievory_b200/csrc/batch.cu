@@ -1405,11 +1405,15 @@ static thv_status fallback_single(thv_graph *g, const uint32_t *src, uint32_t k,
   return THV_OK;
 }
 
+// What a tuned configuration is kept by.  The number counts the kernel's ways
+// of splitting work, so that a file's lines from an earlier one are not used;
+// the window stands for the weights (0 for BFS).
 static std::string tune_key(const thv_graph *g, bool sssp) {
-  char buf[160];
-  snprintf(buf, sizeof(buf), "%s3 nv=%llu ne=%llu esz=%u resident=%llu blocks=%zu sms=%d",
+  char buf[192];
+  snprintf(buf, sizeof(buf), "%s4 nv=%llu ne=%llu esz=%u resident=%llu blocks=%zu sms=%d window=%u",
            sssp ? "sssp" : "bfs", (unsigned long long)g->nv, (unsigned long long)g->ne, g->esz,
-           (unsigned long long)g->plan.resident_edge_bytes, g->plan.blocks.size(), g->num_sms);
+           (unsigned long long)g->plan.resident_edge_bytes, g->plan.blocks.size(), g->num_sms,
+           sssp ? ms_delta(g) : 0u);
   return buf;
 }
 
