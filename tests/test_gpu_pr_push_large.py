@@ -1,8 +1,9 @@
-"""Push PageRank on resident graphs of 8 M edges and more, which take a tile
-per CTA instead of one per warp, against the FP64 oracle: 4-byte ids, packed
-weights and pairs, with hubs above the 1,024 edges from which a row is split,
-empty rows and vertices without out-edges (reference: src/pr/pr_kernels.cu
-:504-681, :846-860).  Tolerance: contributions are rounded to FP32 once per
+"""Push PageRank on resident graphs of more than three warp tiles per warp
+(3.4 M edges or 909 K vertices on 148 SMs), which take a tile per CTA instead
+of one per warp, against the FP64 oracle: 4-byte ids, packed weights and
+pairs, with hubs above the 1,024 edges from which a row is split, empty rows
+and vertices without out-edges (reference: src/pr/pr_kernels.cu :504-681,
+:846-860).  Tolerance: contributions are rounded to FP32 once per
 iteration (6e-8 relative) and contracted by 0.85, so 20 iterations stay below
 4.1e-7 + 6e-8; 1e-6 is the engine's bound.
 """
@@ -42,3 +43,17 @@ def test_resident_push(T, O, graphs, name, fmt):
         for _ in range(2):
             got, _ = g.run("pr_push", pr_iters=20)
             assert float(np.max(np.abs(got - want) / want)) <= 1e-6
+
+
+@pytest.mark.parametrize("n,m", [(909_311, 400_000), (909_600, 400_000), (70_001, 3_409_800), (70_001, 3_410_500)])
+def test_around_the_line(T, O, n, m):
+    """Vertices or edges just below and above the line, mostly empty rows."""
+    rng = np.random.default_rng(n + m)
+    src = np.sort(rng.integers(0, n, m) // 3 * 3 % n)
+    off = np.concatenate([[0], np.cumsum(np.bincount(src, minlength=n))]).astype(np.uint64)
+    c = O.CSR(off, rng.integers(0, n, m).astype(np.uint32))
+    want = O.pagerank(c, 20)
+    with T.Graph.from_arrays(c.off, c.adj, "csr") as g:
+        assert g.plan()["host_edge_bytes"] == 0
+        got, _ = g.run("pr_push", pr_iters=20)
+    assert float(np.max(np.abs(got - want) / want)) <= 1e-6

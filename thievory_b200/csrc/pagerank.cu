@@ -11,10 +11,11 @@
 //
 // Every iteration streams all edges.  A warp (or a CTA: push on large
 // resident graphs) takes one tile, consecutive vertices inside one edge
-// block with at most 480 (4,096) edges, reads the tile's adjacency with 16-byte vector loads -- full 128-byte lines whether the
-// block is in HBM or read zero-copy from pinned host memory -- and gathers
-// (pull) or scatters (push) per edge.  Per-vertex sums are FP64; stored ranks and
-// contributions are FP32.
+// block with at most 480 (4,096) edges, reads the tile's adjacency with
+// 16-byte vector loads -- full 128-byte lines whether the block is in HBM or
+// read zero-copy from pinned host memory -- and gathers (pull) or scatters
+// (push) per edge.  Per-vertex sums are FP64; stored ranks and contributions
+// are FP32.
 // Pull fuses the rank update into the gather: a vertex's sum is complete
 // inside its tile, except high-degree vertices cut into parts, whose last
 // part (atomic counter) finishes the update.
@@ -375,15 +376,27 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
 // CTAs per SM fill the reduction units; more only queue behind them (RMAT
 // 4.2 M vertices, resident: 1 CTA 574 us per iteration, 2 438, 3 438, 4 485).
 //
-// Per iteration against pr_push_cta_kernel: 3,000 vertices 21.4 -> 13.0 us,
-// 262 K (4.1 M edges) 56.2 -> 50.8; with half the edges over the link, 262 K
-// 359 -> 336 us and 3 M vertices (35 M edges) 1,562 -> 1,520 us (loads of
-// whole lines: 46.9 -> 48.2 GB/s over the link).  Resident from 12 M edges up it
-// is 438 us against 460 or 136 against 129, depending on where the hubs' sums
-// fall: one L2 slice at 94% of its requests bounds both, so those keep the
-// CTA kernel.
+// With host-resident edges this kernel is chosen throughout, for its loads of
+// whole lines over the link: half of the edges on the host, per iteration
+// against pr_push_cta_kernel, 262 K vertices 359 -> 336 us, 3 M (35 M edges)
+// 1,562 -> 1,520 (46.9 -> 48.2 GB/s).
+//
+// Resident graphs take it while there are at most kPushWarpTiles tiles per
+// warp: with more, the reduction units bound both kernels and two CTAs per SM
+// bring fewer of them than the CTA kernel's eight.  CTA and warp tiles, us per
+// iteration, RMAT and uniform:
+//   50 K vertices,  2 M edges (1.8 tiles a warp)  37.2  30.6    31.3  24.4
+//   200 K,          2 M       (1.8)               40.4  37.6    34.3  28.4
+//   200 K,          2.8 M     (2.5)               45.6  44.2    38.4  33.3
+//   400 K,          3.2 M     (2.8)               50.2  49.6    39.3  37.6
+//   1 M,            1 M       (3.3)               37.9  49.8    35.6  44.4
+//   250 K,          4 M       (3.5)               54.8  51.8    39.7  41.5
+//   1 M,            4 M       (3.5)               61.0  62.0    47.9  52.2
+//   450 K,          7 M       (6)                 71.4  70.8    52.1  61.7
+//   1 M,            16 M      (14)                 125   125     100   118
+//   4.2 M,          66 M      (58)                 461   466     398   414
 constexpr int kPushCtas = 2;
-constexpr uint64_t kPushWarpEdges = 8ull << 20;
+constexpr uint64_t kPushWarpTiles = 3;
 struct PushWarp {
   float4 x[kSlots / 4];  // source contribution of each slot
   float c[kRows];        // and of each row
@@ -476,8 +489,8 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_push_kernel(PrArgs a) {
   }
 }
 
-// Push with a tile per CTA, staged in shared memory: resident graphs of at
-// least kPushWarpEdges edges.
+// Push with a tile per CTA, staged in shared memory: resident graphs of more
+// than kPushWarpTiles warp tiles per warp.
 template <int ESZ>
 __global__ void __launch_bounds__(kPrThreads) pr_push_cta_kernel(PrArgs a) {
   __shared__ __align__(16) uint32_t s_e[kStageEdges * (ESZ / 4) + 16];
@@ -558,8 +571,9 @@ __global__ void pr_init(PrArgs a, float *c0) {
 // one, which took longer than a resident run's 20 iterations (4.2 M
 // vertices: 8.5 ms after 9.1 ms of iterations).  Widened here, the ranks
 // cross the link as twice the bytes but straight into the caller's buffer
-// (33.5 MB, 0.6 ms; the whole call 17.7 -> 9.7 ms); the two contribution arrays, which nothing reads
-// between runs, hold exactly one half each, so no memory is added.
+// (33.5 MB, 0.6 ms; the whole call 17.7 -> 9.7 ms); the two contribution
+// arrays, which nothing reads between runs, hold exactly one half each, so no
+// memory is added.
 __global__ void pr_widen(const float *rank, uint64_t nv, uint64_t half, double *lo, double *hi) {
   for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < half;
        i += (uint64_t)gridDim.x * blockDim.x) {
@@ -1024,8 +1038,12 @@ thv_status run_pagerank(thv_graph *g, thv_algo algo, const thv_run_opts *o,
   const uint32_t iters = o && o->pr_iters ? o->pr_iters : 20u;
   const double damping = o && o->pr_damping > 0 ? o->pr_damping : 0.85;
   THV_TRY(ensure_plan(g));
-  const PrTileKind kind =
-      push && g->plan.host_edge_bytes == 0 && g->ne >= kPushWarpEdges ? kCtaTiles : kWarpTiles;
+  const uint64_t warps = (uint64_t)kPushCtas * g->num_sms * kPrWarps;
+  const uint64_t warp_tiles =
+      std::max(g->ne / kTileShape[kWarpTiles].edges, g->nv / kTileShape[kWarpTiles].verts);
+  const PrTileKind kind = push && g->plan.host_edge_bytes == 0 && warp_tiles > kPushWarpTiles * warps
+                              ? kCtaTiles
+                              : kWarpTiles;
   THV_TRY(build_tiles(g, kind));
   const PrTiles &tiles = g->plan.tiles[kind];
   THV_TRY(ensure_pr_state(g, push, iters, false, tiles));
