@@ -47,7 +47,9 @@ struct PrArgs {
   uint32_t ntiles, nv, it;
   uint32_t wshift;  // packed weighted edges: the id is e >> wshift
   uint32_t last;    // last iteration
-  uint32_t draw;    // pull: tiles a warp draws at a time
+  uint32_t draw;    // warp tiles: tiles a warp draws at a time
+  uint32_t first;   // warp tiles: warps of a CTA with tiles of a round
+  uint32_t fixed;   // warp tiles: tiles handed out by place
   double damping, inv_n;
 };
 
@@ -204,25 +206,47 @@ __device__ __forceinline__ void tile_rows(const PrArgs &a, const PrTile &t, uint
   }
 }
 
-// Tiles from the iteration's counter, a.draw at a time per warp: the tile
-// after ti (ask before the work on ti that hides the draw, take after it).
+// Tiles, a.draw at a time per warp.  The first a.fixed are handed out by place,
+// in rounds in which the warps of a CTA stand side by side (a.first of them),
+// the rest from the iteration's counter: ask before the work on tile ti, which
+// hides the draw, and take the tile after it.
+//
+// Resident graphs have one such round and draw the rest, which evens out best.
+// With host-resident edges all tiles go by place, so that a CTA reads 16 KB
+// stretches: while warps anywhere on the GPU drew neighbouring 2 KB tiles, an
+// iteration took up to twice its time, the more so the more edges the rows
+// have, and by how the host's pages happened to lie.  All edges on the host,
+// us per iteration on one box, four graphs each: tiles drawn, by place, and
+// (before there were warp tiles) a 16 KB tile per CTA; the link alone takes
+// 155, 466, 1,390 and 3,730:
+//   uniform  50 K vertices,  2 M edges   361-479      174-238      218-226
+//   uniform 100 K,           6 M         500-572      494-528      546-612
+//   uniform 300 K,          18 M       1,753-1,809  1,470-1,494  1,542-1,587
+//   uniform 600 K,          48 M       4,224-4,462  3,879-3,915  4,020-4,063
+//   RMAT    300 K,          12 M         886-900      891-915      968-1,007
+// RMAT of 1.5 M vertices, 60% of 32 M edges: 2,696, 2,715 and 2,800.
 struct TileDraw {
   uint32_t left, drawn;
 };
+__device__ __forceinline__ uint32_t tile_round(const PrArgs &a) { return gridDim.x * a.first * a.draw; }
 __device__ __forceinline__ uint32_t first_tile(const PrArgs &a, TileDraw &d) {
-  uint32_t ti = 0;
-  if (lane_id() == 0) ti = atomicAdd(a.tile_ctr + a.it, a.draw);
+  const uint32_t w = threadIdx.x >> 5;
   d.left = a.draw;
-  return __shfl_sync(kFull, ti, 0);
+  return w < a.first ? (blockIdx.x * a.first + w) * a.draw : a.ntiles;
 }
-__device__ __forceinline__ void ask_tile(const PrArgs &a, TileDraw &d) {
+__device__ __forceinline__ uint32_t next_fixed(const PrArgs &a, uint32_t ti) {
+  return ti + 1 - a.draw + tile_round(a);  // ti is the last of its draw
+}
+__device__ __forceinline__ void ask_tile(const PrArgs &a, TileDraw &d, uint32_t ti) {
   d.drawn = 0;
-  if (d.left == 1 && lane_id() == 0) d.drawn = atomicAdd(a.tile_ctr + a.it, a.draw);
+  if (d.left == 1 && lane_id() == 0 && next_fixed(a, ti) >= a.fixed)
+    d.drawn = a.fixed + atomicAdd(a.tile_ctr + a.it, a.draw);
 }
 __device__ __forceinline__ uint32_t take_tile(const PrArgs &a, TileDraw &d, uint32_t ti) {
   if (--d.left) return ti + 1;
   d.left = a.draw;
-  return __shfl_sync(kFull, d.drawn, 0);
+  const uint32_t next = next_fixed(a, ti);
+  return next < a.fixed ? next : __shfl_sync(kFull, d.drawn, 0);
 }
 
 struct PullWarp {
@@ -262,7 +286,7 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
     tile_words<4>(sp, 0, q);
   }
   while (ti < a.ntiles) {
-    ask_tile(a, draw);
+    ask_tile(a, draw, ti);
     const uint32_t p0 = sp.p0, p1 = p0 + (uint32_t)(t.eend - t.ebegin);
     const uint32_t nrows = t.vend - t.vbegin;
     if (!t.split) tile_rows(a, t, p0, s.rows);
@@ -375,6 +399,9 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
 // FP64 reductions in flight per lane while the next tile's ids load.  Two
 // CTAs per SM fill the reduction units; more only queue behind them (RMAT
 // 4.2 M vertices, resident: 1 CTA 574 us per iteration, 2 438, 3 438, 4 485).
+// With host-resident edges the link is far from filling them, and four CTAs
+// leave fewer rounds of tiles to drift apart (uniform 50 K vertices, 2 M edges
+// on the host: 2 CTAs 176-287 us, 4 174-214; 100 K, 6 M: 498-551 and 499-515).
 //
 // With host-resident edges this kernel is chosen throughout, for its loads of
 // whole lines over the link: half of the edges on the host, per iteration
@@ -395,7 +422,7 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
 //   450 K,          7 M       (6)                 71.4  70.8    52.1  61.7
 //   1 M,            16 M      (14)                 125   125     100   118
 //   4.2 M,          66 M      (58)                 461   466     398   414
-constexpr int kPushCtas = 2;
+constexpr int kPushCtas = 2, kPushHostCtas = 4;
 constexpr uint64_t kPushWarpTiles = 3;
 struct PushWarp {
   float4 x[kSlots / 4];  // source contribution of each slot
@@ -421,7 +448,7 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_push_kernel(PrArgs a) {
     tile_words<ESZ>(sp, 0, qn);
   }
   while (ti < a.ntiles) {
-    ask_tile(a, draw);
+    ask_tile(a, draw, ti);
     const PrTile c = t;
     const TileSpan cs = sp;
     const uint32_t p0 = cs.p0, p1 = p0 + (uint32_t)(c.eend - c.ebegin);
@@ -914,9 +941,10 @@ template <int ESZ>
 static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, PrTileKind kind, uint32_t iters,
                              cudaStream_t st, uint32_t &launches) {
   PrState *p = g->ps;
+  const bool host = g->plan.host_edge_bytes > 0;
   int bpsm = 0;
   if (push && kind == kWarpTiles)
-    bpsm = kPushCtas;
+    bpsm = host ? kPushHostCtas : kPushCtas;
   else if (push)
     THV_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bpsm, pr_push_cta_kernel<ESZ>, kPrThreads, 0));
   else
@@ -925,7 +953,10 @@ static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, PrTileKind kind
   const int ugrid = std::max(1, std::min<int>(g->num_sms * 8, (int)((g->nv + kPrThreads - 1) / kPrThreads)));
   // several tiles per draw only while every warp still draws often enough
   // for the last ones to even out
-  a.draw = std::min(4u, std::max(1u, a.ntiles / (16u * (uint32_t)grid * kPrWarps)));
+  const uint32_t warps = (uint32_t)grid * kPrWarps;
+  a.draw = host ? 1u : std::min(4u, std::max(1u, a.ntiles / (16u * warps)));
+  a.first = std::min((uint32_t)kPrWarps, (a.ntiles + (uint32_t)grid - 1) / (uint32_t)grid);
+  a.fixed = (host ? (a.ntiles + warps - 1) / warps : 1u) * (uint32_t)grid * a.first * a.draw;
   for (uint32_t it = 0; it < iters; it++) {
     a.it = it;
     a.last = it + 1 == iters;
