@@ -103,6 +103,7 @@ struct MsArgs {
   MsCtrl *ctrl;
   const uint32_t *sources;  // [k, source 0, ..., source k-1]
   unsigned long long timeout_ns;
+  uint32_t host_lists;  // some edges are host-resident
   uint32_t nblk, nv, ngroups, max_iters;
   // degree buckets: [1, small_deg) in groups of gsmall vertices per warp,
   // [small_deg, mid_deg) in groups of gmid, the rest in chunk-edge items
@@ -335,17 +336,22 @@ __device__ __forceinline__ void ms_sssp_item(const MsArgs &a, uint32_t ring, uin
 }
 
 // Splits the pending sources f (lane = vertex v0 + lane, vertices wd) by
-// their distance: take holds those below thr, keep the rest, kmin the least
-// kept distance.  Each half-warp reads one vertex's whole row, 16 bytes per
-// lane (the layout of ms_sssp_item), kSplitPer rows in flight per half-warp;
-// ballots turn the lanes' comparisons into the vertex's mask.  (One lane per
-// vertex, reading its pending sources' words one by one, fetched a 32-byte
-// sector per word: eight times the row.)
-constexpr int kSplitPer = 4;
-__device__ __forceinline__ void ms_split_pending(const MsArgs &a, uint32_t v0, uint32_t wd,
-                                                 unsigned long long f, uint32_t thr,
-                                                 unsigned long long &take, unsigned long long &keep,
-                                                 uint32_t &kmin) {
+// their distance: take holds those below thr, kmin the least of the others.
+//
+// Vertices with many pending sources: each half-warp reads one vertex's whole
+// row, 16 bytes per lane (the layout of ms_sssp_item), kSplitPer rows in
+// flight per half-warp; ballots turn the lanes' comparisons into the vertex's
+// mask.  (One lane per vertex, reading its pending sources' words one by one,
+// fetched a 32-byte sector per word: up to eight times the row.)  Vertices
+// with few (kSplitFew): their lane reads the words, a sector each, which are
+// fewer than the row's eight.  Rows throughout, and words up to 8 sources:
+// uniform 3 M vertices, 48 M edges, groups of 8 sources 65.3 and 63.3 ms, of 2
+// 28.5 and 26.7 (words throughout 62.7 and 26.9); RMAT 1 M, 64 sources 4.85
+// and 4.83 (5.78).  Up to 4 sources measured the same within 1%.
+constexpr int kSplitPer = 4, kSplitFew = 8;
+__device__ __forceinline__ void ms_split_rows(const MsArgs &a, uint32_t v0, uint32_t wd,
+                                              unsigned long long f, uint32_t thr,
+                                              unsigned long long &take, uint32_t &kmin) {
   const unsigned lane = lane_id(), hl = lane & 15u, half = lane >> 4;
   for (uint32_t m = wd; m;) {
     int own[kSplitPer][2];  // the two vertices of each step (-1: none)
@@ -381,7 +387,27 @@ __device__ __forceinline__ void ms_split_pending(const MsArgs &a, uint32_t v0, u
       if ((int)lane == own[k][1]) take = hi;
     }
   }
-  keep = f & ~take;
+}
+// One vertex's, by its lane: four loads in flight.
+__device__ __forceinline__ void ms_split_words(const uint32_t *dv, unsigned long long f, uint32_t thr,
+                                               unsigned long long &take, uint32_t &kmin) {
+  while (f) {
+    int s[4];
+    uint32_t d[4];
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      s[k] = f ? __ffsll((long long)f) - 1 : -1;
+      f &= f - 1;
+    }
+#pragma unroll
+    for (int k = 0; k < 4; k++) d[k] = s[k] >= 0 ? ldcg(dv + row_pos((uint32_t)s[k])) : 0u;
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      if (s[k] < 0) continue;
+      if (d[k] < thr) take |= 1ull << s[k];
+      else kmin = min(kmin, d[k]);
+    }
+  }
 }
 
 // masks with at most this many sources relax lane-per-edge instead
@@ -557,7 +583,10 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
   }
   bool yielded = false;
   unsigned wpw = 32;
-  while (wpw > 1 && a.ngroups * (32u / wpw) < nwarps) wpw >>= 1;
+  if (OP == MS_SSSP && a.host_lists)
+    while (wpw > 1 && a.ngroups * (64u / wpw) <= nwarps) wpw >>= 1;
+  else
+    while (wpw > 1 && a.ngroups * (32u / wpw) < nwarps) wpw >>= 1;
   for (;; ++iter) {
     // live groups return here, between iterations: every block has passed
     // the previous iteration's last barrier, and the counter slot of this
@@ -595,6 +624,13 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
     // sources took, before and after (RMAT, edge factor 16): SSSP 3,000
     // vertices 3,026 and 520 us, 150,000 4,587 and 1,642, 2.1 M 11,686 and
     // 10,537; BFS 3,000 524 and 174, 262 K 745 and 566, 4.2 M 6,616 and 6,465.
+    // The words of all vertices fit one round of the warps, or up to two: the
+    // shorter one leaves no warp without words.  SSSP with host-resident edges
+    // takes the single round: in two, vertices of the second half enter the
+    // queues last, and where the host's blocks lie there the link is idle
+    // until then (40% in HBM, one and up to two rounds: RMAT 2 M vertices
+    // 10.6 and 11.8 ms, groups of 8 13.4 and 15.4; 4 M 12.1 and 12.8; all on
+    // the host, 2 M, 15.3 and 14.9; BFS 2 M 7.3 and 7.2).
     unsigned long long my_edges = 0, my_hbm = 0, my_link = 0, my_pairs = 0, my_keep = 0;
     uint32_t my_min = 0xFFFFFFFFu;
     for (unsigned g = gwarp; g < a.ngroups * (32u / wpw); g += nwarps) {
@@ -618,8 +654,18 @@ __global__ void __launch_bounds__(THREADS, 1024 / THREADS) ms_kernel(MsArgs a) {
         unsigned long long take = 0, keep = 0;
         uint32_t kmin = 0xFFFFFFFFu;
         const unsigned long long f = act ? ldcg(a.front + v) : 0ull;
-        if (OP == MS_BFS) take = f;
-        else ms_split_pending(a, (wbase + j) * 32u, wd, f, thr, take, keep, kmin);
+        if (OP == MS_BFS) {
+          take = f;
+        } else {
+          const bool few = act && __popcll(f) <= kSplitFew;
+          const unsigned rows = wd & ~__ballot_sync(kFull, few);
+          if (rows) ms_split_rows(a, (wbase + j) * 32u, rows, few ? 0ull : f, thr, take, kmin);
+          if (few) {
+            take = 0;
+            ms_split_words(a.dist + (size_t)v * kMsWidth, f, thr, take, kmin);
+          }
+          keep = f & ~take;
+        }
         if (act) a.front[v] = keep;
         const unsigned km = __ballot_sync(kFull, keep != 0);
         if (OP == MS_SSSP) {
@@ -1499,6 +1545,7 @@ static MsArgs ms_args(thv_graph *g, BatchState *b, uint32_t timeout_ms) {
   a.nblk = (uint32_t)g->plan.blocks.size();
   a.nv = (uint32_t)g->nv;
   a.ngroups = b->ngroups;
+  a.host_lists = g->plan.host_edge_bytes > 0;
   a.max_iters = (uint32_t)std::min<uint64_t>(g->nv + 2, 0x7FFFFFF0ull) * 2 + 8;
   return a;
 }
