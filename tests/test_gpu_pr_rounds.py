@@ -1,7 +1,8 @@
 """PageRank over many rounds of warp tiles, against the FP64 oracle.
 
-With host-resident edges tiles are handed out by place; resident graphs draw
-them after the first round, several at a time from 152 K tiles.  A tile has at
+With host-resident edges tiles are handed out by place, half of them from 33
+rounds; resident graphs draw them after the first round, several at a time
+from 152 K tiles.  A tile has at
 most 128 rows, so many rows with few edges reach each of these, with the last
 round full, nearly empty and in between (reference:
 src/pr/pr_kernels.cu:23-160, :504-681).  Tolerance: contributions are rounded
@@ -41,12 +42,18 @@ def test_rounds(T, O, n, m, budget):
     assert float(np.max(np.abs(got - want) / want)) <= 1e-6
 
 
-def test_several_tiles_per_draw(T, O):
+@pytest.mark.parametrize("budget", [0.0, 1.0])
+def test_many_rounds(T, O, budget):
     n, m = 20_000_001, 600_000
     off, adj = sparse(O, n, m)
     od = np.bincount(adj, minlength=n).astype(np.uint32)
     want = O.pagerank_csc(off, adj, od, 3)
     with T.Graph.from_arrays(off, adj, "csc", outdeg=od) as g:
-        g.plan()
+        g.plan(int(budget * g.ne * 4))
         got, _ = g.run("pr_pull", pr_iters=3)
+    assert float(np.max(np.abs(got - want) / want)) <= 1e-6
+    want = O.pagerank(O.CSR(off, adj), 3)
+    with T.Graph.from_arrays(off, adj, "csr") as g:
+        g.plan(int(budget * g.ne * 4), small_list_degree=1)
+        got, _ = g.run("pr_push", pr_iters=3)
     assert float(np.max(np.abs(got - want) / want)) <= 1e-6

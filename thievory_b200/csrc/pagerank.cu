@@ -212,8 +212,8 @@ __device__ __forceinline__ void tile_rows(const PrArgs &a, const PrTile &t, uint
 // hides the draw, and take the tile after it.
 //
 // Resident graphs have one such round and draw the rest, which evens out best.
-// With host-resident edges all tiles go by place, so that a CTA reads 16 KB
-// stretches: while warps anywhere on the GPU drew neighbouring 2 KB tiles, an
+// With host-resident edges all tiles of up to kPlacedRounds rounds go by place,
+// and half of more, so that a CTA reads 16 KB stretches: while warps anywhere on the GPU drew neighbouring 2 KB tiles, an
 // iteration took up to twice its time, the more so the more edges the rows
 // have, and by how the host's pages happened to lie.  All edges on the host,
 // us per iteration on one box, four graphs each: tiles drawn, by place, and
@@ -224,7 +224,12 @@ __device__ __forceinline__ void tile_rows(const PrArgs &a, const PrTile &t, uint
 //   uniform 300 K,          18 M       1,753-1,809  1,470-1,494  1,542-1,587
 //   uniform 600 K,          48 M       4,224-4,462  3,879-3,915  4,020-4,063
 //   RMAT    300 K,          12 M         886-900      891-915      968-1,007
-// RMAT of 1.5 M vertices, 60% of 32 M edges: 2,696, 2,715 and 2,800.
+// RMAT of 1.5 M vertices, 60% of 32 M edges: 2,696, 2,715 and 2,800.  Over many
+// rounds the warps drift apart anyway and uneven tiles add up: push of RMAT 67
+// M vertices, half on the host, 480 rounds, 44.6 ms with tiles or half of them
+// drawn and 46.1 with all by place (45.9 with 16 KB tiles per CTA); uniform
+// graphs of 40 and more rounds measure the same either way.
+constexpr uint32_t kPlacedRounds = 32;
 struct TileDraw {
   uint32_t left, drawn;
 };
@@ -956,7 +961,8 @@ static thv_status pr_iterate(thv_graph *g, PrArgs &a, bool push, PrTileKind kind
   const uint32_t warps = (uint32_t)grid * kPrWarps;
   a.draw = host ? 1u : std::min(4u, std::max(1u, a.ntiles / (16u * warps)));
   a.first = std::min((uint32_t)kPrWarps, (a.ntiles + (uint32_t)grid - 1) / (uint32_t)grid);
-  a.fixed = (host ? (a.ntiles + warps - 1) / warps : 1u) * (uint32_t)grid * a.first * a.draw;
+  const uint32_t rounds = (a.ntiles + warps - 1) / warps;
+  a.fixed = (host ? rounds <= kPlacedRounds ? rounds : rounds / 2 : 1u) * (uint32_t)grid * a.first * a.draw;
   for (uint32_t it = 0; it < iters; it++) {
     a.it = it;
     a.last = it + 1 == iters;
