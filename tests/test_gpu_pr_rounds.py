@@ -1,8 +1,7 @@
 """PageRank over many rounds of warp tiles, against the FP64 oracle.
 
-With host-resident edges tiles are handed out by place, half of them from 33
-rounds; resident graphs draw them after the first round, several at a time
-from 152 K tiles.  A tile has at
+With host-resident edges tiles are handed out by place; resident graphs draw
+them after the first round, several at a time from 152 K tiles.  A tile has at
 most 128 rows, so many rows with few edges reach each of these, with the last
 round full, nearly empty and in between (reference:
 src/pr/pr_kernels.cu:23-160, :504-681).  Tolerance: contributions are rounded

@@ -207,29 +207,32 @@ __device__ __forceinline__ void tile_rows(const PrArgs &a, const PrTile &t, uint
 }
 
 // Tiles, a.draw at a time per warp.  The first a.fixed are handed out by place,
-// in rounds in which the warps of a CTA stand side by side (a.first of them),
-// the rest from the iteration's counter: ask before the work on tile ti, which
-// hides the draw, and take the tile after it.
+// in rounds: the first warps of all CTAs take a round's first tiles, then the
+// second warps, and so on (a.first of them).  The rest come from the
+// iteration's counter: ask before the work on tile ti, which hides the draw,
+// and take the tile after it.
 //
 // Resident graphs have one such round and draw the rest, which evens out best.
 // With host-resident edges all tiles of up to kPlacedRounds rounds go by place,
-// and half of more, so that a CTA reads 16 KB stretches: while warps anywhere on the GPU drew neighbouring 2 KB tiles, an
-// iteration took up to twice its time, the more so the more edges the rows
-// have, and by how the host's pages happened to lie.  All edges on the host,
-// us per iteration on one box, four graphs each: tiles drawn, by place, and
-// (before there were warp tiles) a 16 KB tile per CTA; the link alone takes
-// 155, 466, 1,390 and 3,730:
-//   uniform  50 K vertices,  2 M edges   361-479      174-238      218-226
-//   uniform 100 K,           6 M         500-572      494-528      546-612
-//   uniform 300 K,          18 M       1,753-1,809  1,470-1,494  1,542-1,587
-//   uniform 600 K,          48 M       4,224-4,462  3,879-3,915  4,020-4,063
-//   RMAT    300 K,          12 M         886-900      891-915      968-1,007
-// RMAT of 1.5 M vertices, 60% of 32 M edges: 2,696, 2,715 and 2,800.  Over many
-// rounds the warps drift apart anyway and uneven tiles add up: push of RMAT 67
-// M vertices, half on the host, 480 rounds, 44.6 ms with tiles or half of them
-// drawn and 46.1 with all by place (45.9 with 16 KB tiles per CTA); uniform
-// graphs of 40 and more rounds measure the same either way.
-constexpr uint32_t kPlacedRounds = 32;
+// and half of more.  The order of reads over the link counts: where all warps
+// drew their tiles, and where the warps of a CTA stood side by side, an
+// iteration took up to twice its time on some boxes and for some placements of
+// the host's pages, the more so the more edges the rows have, since early CTAs
+// read one part of the array and late ones another.  In this order the CTAs
+// that start together read all over a round's part of it.  All edges on the
+// host, us per iteration on one box, three graphs each: tiles drawn, the warps
+// of a CTA side by side, this order; a 16 KB tile per CTA (before there were
+// warp tiles) on another box; the link alone takes 155, 466, 1,390 and 3,730:
+//   uniform  50 K vertices,  2 M edges   258-394      213-289      174        202-248
+//   uniform 100 K,           6 M         500-530      498-619      494-495    527-640
+//   uniform 300 K,          18 M       1,713-1,749  1,470-1,494  1,460-1,466  1,542-1,587
+//   uniform 600 K,          48 M       4,245-4,381  3,879-3,915  3,864-3,866  4,020-4,063
+//   RMAT    300 K,          12 M         886-900      890-910      892-900    968-1,007
+// Over very many rounds uneven tiles add up: push of RMAT 67 M vertices, half
+// on the host, 530 rounds, 44.6 ms with tiles or half of them drawn, 46.1 with
+// all by place (45.9 with 16 KB tiles per CTA); RMAT 17 M vertices, 350
+// rounds, 40.6 and 40.7.
+constexpr uint32_t kPlacedRounds = 256;
 struct TileDraw {
   uint32_t left, drawn;
 };
@@ -237,7 +240,7 @@ __device__ __forceinline__ uint32_t tile_round(const PrArgs &a) { return gridDim
 __device__ __forceinline__ uint32_t first_tile(const PrArgs &a, TileDraw &d) {
   const uint32_t w = threadIdx.x >> 5;
   d.left = a.draw;
-  return w < a.first ? (blockIdx.x * a.first + w) * a.draw : a.ntiles;
+  return w < a.first ? (w * gridDim.x + blockIdx.x) * a.draw : a.ntiles;
 }
 __device__ __forceinline__ uint32_t next_fixed(const PrArgs &a, uint32_t ti) {
   return ti + 1 - a.draw + tile_round(a);  // ti is the last of its draw
@@ -405,8 +408,8 @@ __global__ void __launch_bounds__(kPrThreads, 4) pr_pull_kernel(PrArgs a) {
 // CTAs per SM fill the reduction units; more only queue behind them (RMAT
 // 4.2 M vertices, resident: 1 CTA 574 us per iteration, 2 438, 3 438, 4 485).
 // With host-resident edges the link is far from filling them, and four CTAs
-// leave fewer rounds of tiles to drift apart (uniform 50 K vertices, 2 M edges
-// on the host: 2 CTAs 176-287 us, 4 174-214; 100 K, 6 M: 498-551 and 499-515).
+// keep more reads in flight (uniform 200 K vertices, 2 M edges on the host: 2
+// CTAs 180 us, 4 178; RMAT 200 K 173 and 168).
 //
 // With host-resident edges this kernel is chosen throughout, for its loads of
 // whole lines over the link: half of the edges on the host, per iteration
