@@ -296,7 +296,9 @@ typedef struct thv_batch_opts {
    * small_group, mid_group non-zero selects an explicit configuration (the
    * zeros among them take the defaults: mid_degree = small_degree, i.e. no
    * middle bucket; small_group 32; mid_group 4); all zero selects the tuned
-   * or default one. */
+   * or default one.  small_group and chunk_edges are upper bounds: while an
+   * iteration has too few tasks for the GPU's warps, groups of small vertices
+   * shrink and chunks split. */
   uint32_t mid_degree;
   uint32_t small_group;  /* 1..32 */
   uint32_t mid_group;    /* 1..32 */
