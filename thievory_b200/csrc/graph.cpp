@@ -784,9 +784,9 @@ thv_status build_tiles(thv_graph *g, PrTileKind kind) {
     close(b.vend);
   }
   // Interleave host-block and HBM-block tiles in proportion to their edges.
-  // CTAs take tiles in this order from one counter, so the host link stays
-  // busy for the whole iteration while the HBM tiles are done beside it; in
-  // block order the GPU would work through host blocks with HBM idle, then
+  // Tiles are taken in this order, drawn or a round at a time, so the host
+  // link stays busy for the whole iteration while the HBM tiles are done
+  // beside it; in block order the GPU would work through host blocks with HBM idle, then
   // HBM blocks with the link idle.  Results do not depend on the order.
   {
     std::vector<PrTile> host, hbm;

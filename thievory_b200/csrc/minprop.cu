@@ -1853,7 +1853,7 @@ constexpr uint32_t kUfSample = 2;
 // lies in G with about the share of the edges that G's members own, reach.
 // Flat graphs around one planted hub (uniform or grid, the hub's neighbours
 // 1/2 to 1/200 of the vertices) own little more than the hub's share of the
-// vertices and lose by G, up to 1.9 times with host-resident edges (1 M
+// vertices and lose by G, up to 2.2 times with host-resident edges (1 M
 // vertices, 8 M edges, share 1/16, 40% in HBM: 773 us without, 1,299 with;
 // resident 175 and 240); what makes it pay are neighbours that are hubs
 // themselves.  Device us without G, with one sweep and with two, by reach:
